@@ -40,22 +40,23 @@ int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // One 128-body tile of the caller's arrays (a system's tiles start at its
 // first body; its last one may be partial): whether every softening is
 // positive and equal to eps2[0], whether every mass equals the tile's first,
-// the smallest h = eps2 / 2 and the sum of |m|.
+// whether every softening does, the smallest h = eps2 / 2 and the sum of |m|.
 struct TileScan {
     int64_t begin, end;
     int sys;
-    bool pos_eps, same_eps, same_mass;
+    bool pos_eps, same_eps, same_mass, tile_eps;
     double hmin, msum;
 };
 
 void scan_tile(const double* mass, const double* eps2, double e0, TileScan& t) {
-    const double m0 = mass[t.begin];
-    bool pos = true, same_e = true, same_m = true;
+    const double m0 = mass[t.begin], e1 = eps2[t.begin];
+    bool pos = true, same_e = true, same_m = true, tile_e = true;
     double h = 1e300, s[4] = {0.0, 0.0, 0.0, 0.0};
     for (int64_t i = t.begin; i < t.end; ++i) {
         const double e = eps2[i], m = mass[i];
         pos &= e > 0.0;
         same_e &= e == e0;
+        tile_e &= e == e1;
         same_m &= m == m0;
         h = std::min(h, e);
         s[(i - t.begin) & 3] += std::fabs(m);  // four running sums, added pairwise
@@ -63,6 +64,7 @@ void scan_tile(const double* mass, const double* eps2, double e0, TileScan& t) {
     t.pos_eps = pos;
     t.same_eps = same_e;
     t.same_mass = same_m;
+    t.tile_eps = tile_e;
     t.hmin = 0.5 * h;
     t.msum = (s[0] + s[1]) + (s[2] + s[3]);
 }
@@ -76,7 +78,7 @@ std::vector<TileScan> scan_state_tiles(const double* mass, const double* eps2, c
     tiles.reserve(static_cast<size_t>(off[nsys] / kPad + nsys));
     for (int k = 0; k < nsys; ++k)
         for (int64_t b = off[k]; b < off[k + 1]; b += kPad)
-            tiles.push_back(TileScan{b, std::min(b + kPad, off[k + 1]), k, false, false, false, 0.0, 0.0});
+            tiles.push_back(TileScan{b, std::min(b + kPad, off[k + 1]), k, false, false, false, false, 0.0, 0.0});
     const double e0 = eps2[0];
     const unsigned hw = std::thread::hardware_concurrency();
     const int nthreads = off[nsys] < (int64_t(1) << 17) ? 1 : static_cast<int>(std::clamp(hw, 1u, 8u));
@@ -313,6 +315,43 @@ void plan_pair_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, 
                      [](const PairItem& a, const PairItem& b) { return a.cost > b.cost; });
 }
 
+// Work in units of one i block against one j tile.  A chunk's size at any
+// point is a quarter of what is left divided by the CTAs (at most 256 tiles,
+// at least one): few items while much is left, single tiles at the end, so
+// the grid's last round is a fraction of a tile per CTA.  (FP64 passes: 370 ->
+// 130 us at 10,007 bodies, whose 55 block pairs of eight tiles each left most
+// of the 296 CTAs without an item.)  The block's own
+// tiles come with diag_end = i_end in every chunk that holds some of them.
+void plan_pair_tiles(const std::vector<int64_t>& poff, const std::vector<int64_t>& cnt, int ctas, ForcePlan& out) {
+    out.pair_items.clear();
+    out.nslots = 1;
+    constexpr int64_t kPerBlock = kPairBlock / kPad;
+    int64_t left = 0;
+    for (size_t k = 0; k < cnt.size(); ++k) {
+        const int64_t T = (poff[k + 1] - poff[k]) / kPad;
+        for (int64_t b = 0; b < T; b += kPerBlock) left += T - b;
+    }
+    for (size_t k = 0; k < cnt.size(); ++k) {
+        const int64_t T = (poff[k + 1] - poff[k]) / kPad;
+        for (int64_t b = 0; b < T; b += kPerBlock) {
+            for (int64_t t = b; t < T;) {
+                const int64_t c = std::min(std::clamp<int64_t>(left / (4 * std::max(ctas, 1)), 1, 256), T - t);
+                PairItem it{};
+                it.i_begin = static_cast<int>(poff[k] + b * kPad);
+                it.i_end = static_cast<int>(poff[k] + std::min(b + kPerBlock, T) * kPad);
+                it.j_begin = static_cast<int>(poff[k] + t * kPad);
+                it.j_end = static_cast<int>(poff[k] + (t + c) * kPad);
+                it.diag_end = it.i_end;
+                it.real_end = static_cast<int>(poff[k] + cnt[k]);
+                it.cost = static_cast<int>(c);
+                out.pair_items.push_back(it);
+                t += c;
+                left -= c;
+            }
+        }
+    }
+}
+
 }  // namespace khrr
 
 khrr_status khrr_ctx::ensure_plan(int mode) {
@@ -320,8 +359,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
     const bool plain = mode == kModePlain;
     khrr_status st;
     if (mode == kModeF64) {
-        // The symmetric FP64 kernel on the pair plan over 1024-body blocks
-        // (one partial slot per body, FP64 atomics), or with
+        // The symmetric FP64 kernel on the tapered pair plan, or with
         // KHRR_FP64_ONESIDED=1 the one-sided kernel's queue: 512-body i
         // tiles, 128-body j tiles, the j split that fills the last wave of
         // its resident CTAs.
@@ -330,9 +368,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
         const int ctas = sym ? fp64_pair_ctas(sm_count) : fp64_force_ctas(sm_count);
         if (p.valid && p.ctas == ctas && p.f64_pair == sym) return KHRR_OK;
         if (sym) {
-            plan_pair_items(pair_blocks_fixed(poff), cnt, ctas, 0, p);
-            p.nslots = 1;
-            p.sys_split.assign(cnt.size(), 1);
+            plan_pair_tiles(poff, cnt, ctas, p);
             if ((st = cuda(p.d_pair_items.ensure(p.pair_items.size()), "alloc items")) != KHRR_OK) return st;
             if ((st = cuda(cudaMemcpyAsync(p.d_pair_items.p, p.pair_items.data(),
                                            p.pair_items.size() * sizeof(PairItem), cudaMemcpyHostToDevice, stream),
@@ -348,19 +384,23 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
         }
         p.pair = false;
         p.f64_pair = sym;
-        p.threads = sym ? kPairBlock / 4 : 128;
-        p.ipt = sym ? 4 : kF64ITile / 128;
+        p.threads = 128;
+        p.ipt = (sym ? kPairBlock : kF64ITile) / 128;
         p.jt = kPad;
         p.split_req = 0;
         p.ctas = ctas;
-        std::vector<unsigned char> ns(static_cast<size_t>(npad), 0);
-        for (size_t k = 0; k < cnt.size(); ++k)
-            std::fill(ns.begin() + poff[k], ns.begin() + poff[k] + cnt[k], static_cast<unsigned char>(p.sys_split[k]));
-        if ((st = cuda(p.d_nsplit.ensure(ns.size()), "alloc nsplit")) != KHRR_OK) return st;
-        if ((st = cuda(cudaMemcpyAsync(p.d_nsplit.p, ns.data(), ns.size(), cudaMemcpyHostToDevice, stream),
-                       "upload nsplit")) != KHRR_OK)
-            return st;
-        if ((st = cuda(part.ensure(static_cast<size_t>(p.nslots) * npad), "alloc partials")) != KHRR_OK) return st;
+        if (sym) {
+            if ((st = cuda(f64_sums.ensure(8 * static_cast<size_t>(npad)), "alloc sums")) != KHRR_OK) return st;
+        } else {
+            std::vector<unsigned char> ns(static_cast<size_t>(npad), 0);
+            for (size_t k = 0; k < cnt.size(); ++k)
+                std::fill(ns.begin() + poff[k], ns.begin() + poff[k] + cnt[k], static_cast<unsigned char>(p.sys_split[k]));
+            if ((st = cuda(p.d_nsplit.ensure(ns.size()), "alloc nsplit")) != KHRR_OK) return st;
+            if ((st = cuda(cudaMemcpyAsync(p.d_nsplit.p, ns.data(), ns.size(), cudaMemcpyHostToDevice, stream),
+                           "upload nsplit")) != KHRR_OK)
+                return st;
+            if ((st = cuda(part.ensure(static_cast<size_t>(p.nslots) * npad), "alloc partials")) != KHRR_OK) return st;
+        }
         if ((st = cuda(cudaStreamSynchronize(stream), "plan sync")) != KHRR_OK) return st;
         p.valid = true;
         drop_graphs();  // captured graphs may hold the old queue or partial buffer
@@ -470,7 +510,7 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
         return st;
     if (mode == kModeF64 && p.f64_pair) {
         if ((st = cuda(cudaMemsetAsync(queue.p, 0, sizeof(unsigned), stream), "queue reset")) != KHRR_OK) return st;
-        if ((st = cuda(cudaMemsetAsync(part.p, 0, sizeof(double4) * npad, stream), "sums reset")) != KHRR_OK)
+        if ((st = cuda(cudaMemsetAsync(f64_sums.p, 0, 8 * sizeof(double) * npad, stream), "sums reset")) != KHRR_OK)
             return st;
         F64PairArgs a{};
         a.pos = x;
@@ -479,7 +519,10 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
         a.items = p.d_pair_items.p;
         a.n_items = static_cast<int>(p.pair_items.size());
         a.queue = queue.p;
-        a.sums = part.p;
+        a.sums = f64_sums.p;
+        a.npad = npad;
+        a.scale = fx_scale.p;
+        a.tile_class = tile_class64.p;
         if ((st = cuda(launch_fp64_pair(a, acc, phi, std::min(a.n_items, ctas), stream), "FP64 pair kernel")) !=
             KHRR_OK)
             return st;
@@ -557,6 +600,7 @@ StepArgs khrr_ctx::step_args(const ForcePlan& p, double dt) {
     a.npad = npad;
     a.nsplit = p.d_nsplit.p;
     a.fx = p.pair ? fx.p : nullptr;
+    a.f64 = p.f64_pair ? f64_sums.p : nullptr;
     a.fx_scale = fx_scale.p;
     a.n = npad;
     a.dt = dt;
@@ -852,6 +896,7 @@ khrr_status khrr_upload_state(khrr_ctx* c, int64_t n, const double* pos, const d
     if ((st = c->cuda(c->shadow_buf.ensure(5 * np), "alloc shadow")) != KHRR_OK) return st;
     if ((st = c->cuda(c->tile_mass.ensure(np / kPad), "alloc tile masses")) != KHRR_OK) return st;
     if ((st = c->cuda(c->fx_scale.ensure(np / kPad), "alloc tile scales")) != KHRR_OK) return st;
+    if ((st = c->cuda(c->tile_class64.ensure(np / kPad), "alloc tile classes")) != KHRR_OK) return st;
     cudaStream_t s = c->stream;
     for (DevBuf<double>* b : {&c->pos, &c->vel, &c->acc, &c->post, &c->velt, &c->acct})
         cudaMemsetAsync(b->p, 0, 3 * np * sizeof(double), s);
@@ -902,12 +947,15 @@ khrr_status khrr_upload_state(khrr_ctx* c, int64_t n, const double* pos, const d
     bool uniform_new = true, tile_uniform = true;
     std::vector<double> sys_msum(static_cast<size_t>(nsys), 0.0), sys_hmin(static_cast<size_t>(nsys), 1e300);
     std::vector<float> tm(np / kPad, 0.0f);
+    std::vector<double2> tc(np / kPad, make_double2(0.0, -1.0));
     for (const TileScan& t : tiles) {
         uniform_new = uniform_new && t.same_eps;
         tile_uniform = tile_uniform && t.same_mass && t.end - t.begin == kPad;
         sys_msum[t.sys] += t.msum;
         sys_hmin[t.sys] = std::min(sys_hmin[t.sys], t.hmin);
-        tm[(poff[t.sys] + t.begin - off[t.sys]) / kPad] = static_cast<float>(mass[t.begin]);
+        const size_t at = static_cast<size_t>((poff[t.sys] + t.begin - off[t.sys]) / kPad);
+        tm[at] = static_cast<float>(mass[t.begin]);
+        if (t.same_mass && t.tile_eps && t.end - t.begin == kPad) tc[at] = make_double2(mass[t.begin], 0.5 * eps2[t.begin]);
     }
     const bool same_layout = same_offsets && c->uniform == uniform_new &&
                              c->h_uniform == static_cast<float>(0.5 * eps2[0]);
@@ -940,6 +988,9 @@ khrr_status khrr_upload_state(khrr_ctx* c, int64_t n, const double* pos, const d
                  "upload");
     if (st == KHRR_OK)
         st = c->cuda(cudaMemcpyAsync(c->tile_mass.p, tm.data(), tm.size() * sizeof(float), cudaMemcpyHostToDevice, s),
+                     "upload");
+    if (st == KHRR_OK)
+        st = c->cuda(cudaMemcpyAsync(c->tile_class64.p, tc.data(), tc.size() * sizeof(double2), cudaMemcpyHostToDevice, s),
                      "upload");
     if (st == KHRR_OK)
         st = c->cuda(launch_pack(c->pos.p, c->mass.p, c->eps2.p, c->npad, c->npad, c->shadow(), s), "pack");

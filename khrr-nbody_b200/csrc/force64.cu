@@ -129,43 +129,172 @@ __global__ void __launch_bounds__(NT, kMinCtas) fp64_force_kernel(const F64Args 
 
 // The symmetric form of the same sums (the default FP64 pass): every
 // unordered pair of a system evaluated once for both bodies, on the FP32
-// pair kernel's work plan (1024-body blocks, a block row cut into chunks,
-// the block's own tiles one-sided).  A CTA holds its i block in registers
-// (256 threads x 4 bodies) and streams the chunk's j tiles of 128 bodies
-// through a double-buffered shared-memory tile; the reaction on a j body is
-// summed across a warp by handing it from lane to lane (lane l evaluates
-// body (l + s) mod 32 of a 32-body sub-chunk at step s and passes its running
-// reaction to lane l - 1), then across the 8 warps in shared memory, and
-// added with FP64 atomics into the body's sums (one partial slot), as are
-// the i block's sums at the item's end.  Per unordered pair: d (3 sub),
-// r^2 (1 add, 3 fma), rsqrt, r^-3 (2 mul), m_j r^-3 and m_i r^-3 (2 mul),
-// the two sides (6 fma; +2 fma for the potential).  The sums are FP64
-// throughout; their order differs from the reference's j loop (and between
-// runs, through the atomics) only at the level of FP64 rounding.
-#ifndef KHRR_F64P_NT
-#define KHRR_F64P_NT 256
-#endif
-#ifndef KHRR_F64P_UNROLL
-#define KHRR_F64P_UNROLL 2
-#endif
-#ifndef KHRR_F64P_CTAS
-#define KHRR_F64P_CTAS 2
-#endif
-constexpr int PNT = KHRR_F64P_NT;         // threads per CTA
-constexpr int kF64PUnroll = KHRR_F64P_UNROLL;
-constexpr int PK = kPairBlock / PNT;      // i bodies per thread (4)
+// pair kernel's work plan (1024-body blocks, a block row cut into chunks of
+// 128-body tiles, the block's own tiles one-sided).  A CTA holds its i block
+// in registers (128 threads x 8 bodies) and streams the chunk's j tiles of
+// 128 bodies through a double-buffered shared-memory tile; the reaction on a
+// j body is summed across a warp by handing it from lane to lane (lane l
+// evaluates body (l + s) mod 32 of a 32-body sub-chunk at step s and passes
+// its running reaction to lane l - 1), then across the 4 warps in shared
+// memory, and added with FP64 atomics into the body's sums, as are the i
+// block's sums every eighth tile and at the item's end.  The sums are FP64
+// throughout; their order differs from the reference's j loop only at the
+// level of FP64 rounding.
+//
+// A body's sum over the partials is kept in two doubles: every partial is cut at a multiple of the body's grid, coarse enough
+// (2^-51 of the bound on its force) that the upper parts add up without
+// rounding, and the lower parts, below 2^-52 of that bound, add up in the
+// second.  So the number of partials, and the order the atomics land in, do
+// not show in the result: relative RMS error against 80-bit sums 2.4e-16 with
+// one double and chunks of eight tiles, 3.5e-16 with one double and these
+// chunks, 1.0e-16 cut, at 49,152 bodies (5.3e-16, 1.9e-16, 1.6e-16 at 3,072).
+//
+// The kernel is bound by the FP64 pipe (64 lanes per SM and clock), so what
+// counts is FP64 instructions per unordered pair:
+//   * r^-1 and r^-3 from the hardware's reciprocal-square-root seed y0 (one
+//     XU instruction on the upper word, relative error 2^-20) and the
+//     binomial series of (1 - e)^(-1/2) and (1 - e)^(-3/2) in e = 1 - r2 y0^2
+//     (y0^2 is exact, y0 having 21 significant bits), cut after e^2: the
+//     terms left out are 5/16 e^3 and 35/16 e^3, below 2^-55 for |e| < 2^-19.  Six operations for r^-3 (five for r^-1 and two more for
+//     its cube when the potential is wanted too) instead of rsqrt() with its
+//     range handling and two multiplies.
+//   * where the i block has one mass and one softening and so has the j tile
+//     (all but the tiles at a component's border and a ragged end), the
+//     masses leave the pair term (applied once per sum) and h_i + h_j is a
+//     constant: 18 operations per unordered pair (3 sub, 3 fma, 6, 6 fma)
+//     against 21 with per-body masses and softenings.
+// Per pass: 2.24 -> 1.57 ms at 49,152 bodies, 370 -> 130 us at 10,007 (the
+// tapered plan: 55 block pairs left most SMs idle).
+// The series needs r2 well inside the exponent range: tiles whose h or
+// coordinates leave [2^-600, 2^580] and 2^290 in magnitude (or are not
+// numbers) take rsqrt(), which handles every operand.
+// Shape, measured (ms per pass at 131,072 bodies, accelerations / with the
+// potential): 128 threads x 8 bodies, two CTAs per SM, step loop unrolled 8
+// times 10.5 / 14.1, 4 times 10.8 / 13.0, twice 11.1 / 12.9, once 11.5 / 13.0;
+// three CTAs (168 registers) 11.0 / 13.7 (before the cut sums); 256 x 4 11.3 /
+// 12.6.  The kernel before, rsqrt() and per-body masses throughout: 14.5 /
+// 16.0.  What bounds it: DFMA reads three 64-bit registers, and the register
+// file delivers one a cycle (3.05 cycles for three different operands
+// against 2.05 for two, measured on plain chains), so a pair costs 43
+// register-read cycles where its 18 operations would issue in 36; the pass
+// above takes 45.
+constexpr int PNT = 128;                  // threads per CTA
+constexpr int kF64PUnroll = 8, kF64PUnrollPhi = 2;
+constexpr int PK = kPairBlock / PNT;      // i bodies per thread (8)
 constexpr int PJT = kPairTile;            // j bodies per tile (128)
-constexpr int PW = PNT / 32;              // warps (8)
+constexpr int PW = PNT / 32;              // warps (4)
 static_assert(PNT * PK == kPairBlock && PJT == 128 && PJT % 32 == 0 && PNT >= PJT, "pair shapes");
 
-template <bool ACC, bool PHI>
-__global__ void __launch_bounds__(PNT, KHRR_F64P_CTAS) fp64_pair_kernel(const F64PairArgs a) {
+constexpr double kSafePos = 0x1p290, kSafeHMin = 0x1p-600, kSafeHMax = 0x1p580;
+
+__device__ __forceinline__ bool safe_body(double x, double y, double z, double h) {
+    return fabs(x) < kSafePos && fabs(y) < kSafePos && fabs(z) < kSafePos && h > kSafeHMin && h < kSafeHMax;
+}
+
+__device__ __forceinline__ double rsqrt_seed(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+
+// r^-3, and r^-1 where the potential needs it, of a normal r2 (see above).
+template <bool PHI>
+__device__ __forceinline__ void inverse_powers(double r2, double& inv, double& i3) {
+    const double y0 = rsqrt_seed(r2);
+    const double s = y0 * y0;
+    const double e = fma(-r2, s, 1.0);
+    if (PHI) {
+        inv = fma(y0 * e, fma(0.375, e, 0.5), y0);
+        i3 = inv * inv * inv;
+    } else {
+        const double c = s * y0;
+        i3 = fma(c * e, fma(1.875, e, 1.5), c);
+    }
+}
+
+// Adds v into the pair of sums, cut at the grid 2^-52 c / 1.5.
+__device__ __forceinline__ void add_cut(double* upper, int64_t lower, double v, double c) {
+    const double u = (v + c) - c;
+    const double l = v - u;
+    atomicAdd(upper, u);
+    atomicAdd(upper + lower, fabs(v) < 0x1p1000 ? l : 0.0);  // an infinite or overlarge v stays what it is
+}
+constexpr double kCutGrid = 0x1.8p62;  // times a tile's 2^-E (FxScale): 1.5 x 2^52 grids of 2^(10-E)
+
+struct F64Tiles {
+    double x[2][PJT], y[2][PJT], z[2][PJT], m[2][PJT], h[2][PJT];
+};
+
+// One staged tile against the thread's PK bodies.  SYM adds the reactions
+// (jw[c][body] of the warp).  UNI: one mass and softening on either side, the
+// sums without their masses, H = h_i + h_j.  SAFE: the series above.
+template <bool ACC, bool PHI, bool SYM, bool UNI, bool SAFE>
+__device__ __forceinline__ void fp64_pair_tile(const F64Tiles& T, int b, double H, double (*__restrict__ jw)[PJT],
+                                               const double (&xi)[PK], const double (&yi)[PK], const double (&zi)[PK],
+                                               const double (&hi)[PK], const double (&mi)[PK],
+                                               double (&ai)[(ACC ? 3 : 0) + (PHI ? 1 : 0)][PK], int lane) {
     constexpr int NC = (ACC ? 3 : 0) + (PHI ? 1 : 0), CP = NC - 1;
-    __shared__ double tx[2][PJT], ty[2][PJT], tz[2][PJT], tm[2][PJT], th[2][PJT];
+    constexpr int kU = PHI ? kF64PUnrollPhi : kF64PUnroll;
+    const int src = (lane + 1) & 31;
+#pragma unroll 1
+    for (int c0 = 0; c0 < PJT; c0 += 32) {
+        double r[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) r[c] = 0.0;
+#pragma unroll kU
+        for (int s = 0; s < 32; ++s) {
+            const int j = c0 + ((lane + s) & 31);
+            const double xj = T.x[b][j], yj = T.y[b][j], zj = T.z[b][j];
+            const double mj = UNI ? 1.0 : T.m[b][j], hj = UNI ? 0.0 : T.h[b][j];
+#pragma unroll
+            for (int k = 0; k < PK; ++k) {
+                const double dx = xj - xi[k], dy = yj - yi[k], dz = zj - zi[k];
+                double r2 = UNI ? H : hi[k] + hj;
+                r2 = fma(dx, dx, r2);
+                r2 = fma(dy, dy, r2);
+                r2 = fma(dz, dz, r2);
+                double inv = 0.0, i3 = 0.0;
+                if (SAFE) {
+                    inverse_powers<PHI>(r2, inv, i3);
+                } else {
+                    inv = rsqrt(r2);
+                    i3 = inv * inv * inv;
+                }
+                if (ACC) {
+                    const double fi = UNI ? i3 : mj * i3;
+                    const double fj = UNI ? i3 : (SYM ? mi[k] * i3 : 0.0);
+                    ai[0][k] = fma(dx, fi, ai[0][k]);
+                    if (SYM) r[0] = fma(dx, fj, r[0]);
+                    ai[1][k] = fma(dy, fi, ai[1][k]);
+                    if (SYM) r[1] = fma(dy, fj, r[1]);
+                    ai[2][k] = fma(dz, fi, ai[2][k]);
+                    if (SYM) r[2] = fma(dz, fj, r[2]);
+                }
+                if (PHI) {
+                    ai[CP][k] = UNI ? ai[CP][k] + inv : fma(mj, inv, ai[CP][k]);
+                    if (SYM) r[CP] = UNI ? r[CP] + inv : fma(mi[k], inv, r[CP]);
+                }
+            }
+            if (SYM) {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) r[c] = __shfl_sync(0xffffffffu, r[c], src);
+            }
+        }
+        if (SYM) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) jw[c][c0 + lane] = r[c];
+        }
+    }
+}
+
+template <bool ACC, bool PHI>
+__global__ void __launch_bounds__(PNT, 2) fp64_pair_kernel(const F64PairArgs a) {
+    constexpr int NC = (ACC ? 3 : 0) + (PHI ? 1 : 0), CP = NC - 1;
+    __shared__ F64Tiles T;
     __shared__ double jw[PW][NC][PJT];
     __shared__ int s_item;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int src = (lane + 1) & 31;
+    const int64_t lower = 4 * a.npad;  // from a sum's upper part to its lower one
     for (;;) {
         if (tid == 0) s_item = static_cast<int>(atomicAdd(a.queue, 1u));
         __syncthreads();
@@ -174,7 +303,8 @@ __global__ void __launch_bounds__(PNT, KHRR_F64P_CTAS) fp64_pair_kernel(const F6
         const PairItem w = a.items[it];
         // The i bodies (index i_begin + k PNT + tid); lanes past the block's
         // end have no mass (and a positive softening term).
-        double xi[PK], yi[PK], zi[PK], hi[PK], mi[PK], ai[NC][PK];
+        double xi[PK], yi[PK], zi[PK], ai[NC][PK];
+        bool safe_i = true;
 #pragma unroll
         for (int k = 0; k < PK; ++k) {
             const int64_t i = w.i_begin + k * PNT + tid;
@@ -182,14 +312,42 @@ __global__ void __launch_bounds__(PNT, KHRR_F64P_CTAS) fp64_pair_kernel(const F6
             xi[k] = in ? a.pos[3 * i] : 0.0;
             yi[k] = in ? a.pos[3 * i + 1] : 0.0;
             zi[k] = in ? a.pos[3 * i + 2] : 0.0;
-            hi[k] = in ? 0.5 * a.eps2[i] : 1.0;
-            mi[k] = in ? a.mass[i] : 0.0;
+            safe_i = safe_i && safe_body(xi[k], yi[k], zi[k], in ? 0.5 * a.eps2[i] : 1.0);
 #pragma unroll
             for (int c = 0; c < NC; ++c) ai[c][k] = 0.0;
         }
+        // Whether the block is 1024 real bodies of one mass and softening.
+        const double2 ci = a.tile_class[w.i_begin / PJT];
+        bool uni_i = w.i_end - w.i_begin == kPairBlock && ci.y > 0.0;
+        for (int q = 1; uni_i && q < kPairBlock / PJT; ++q) {
+            const double2 cq = a.tile_class[w.i_begin / PJT + q];
+            uni_i = cq.x == ci.x && cq.y == ci.y;
+        }
+        double scale_i = 1.0;  // the mass left out of the sums in ai
+        // The sums so far, times the mass left out of them, into the bodies'
+        // accumulators.
+        auto flush = [&]() {
+#pragma unroll
+            for (int k = 0; k < PK; ++k) {
+                const int64_t i = w.i_begin + k * PNT + tid;
+                if (i < w.i_end && i < w.real_end) {
+                    const FxScale sc = a.scale[i / PJT];
+                    double* u = a.sums + i;
+                    if (ACC) {
+                        const double c = kCutGrid * sc.inv_acc;
+                        add_cut(u, lower, scale_i * ai[0][k], c);
+                        add_cut(u + a.npad, lower, scale_i * ai[1][k], c);
+                        add_cut(u + 2 * a.npad, lower, scale_i * ai[2][k], c);
+                    }
+                    if (PHI) add_cut(u + 3 * a.npad, lower, scale_i * ai[CP][k], kCutGrid * sc.inv_phi);
+                }
+#pragma unroll
+                for (int c = 0; c < NC; ++c) ai[c][k] = 0.0;
+            }
+        };
         const int ntiles = (w.j_end - w.j_begin) / PJT;
         // Register copy of the next tile's body tid (threads < PJT).
-        double nx = 0.0, ny = 0.0, nz = 0.0, nm = 0.0, nh = 0.0;
+        double nx = 0.0, ny = 0.0, nz = 0.0, nm = 0.0, nh = 1.0;
         auto fetch = [&](int t) {
             if (tid < PJT) {
                 const int64_t j = w.j_begin + static_cast<int64_t>(t) * PJT + tid;
@@ -204,60 +362,46 @@ __global__ void __launch_bounds__(PNT, KHRR_F64P_CTAS) fp64_pair_kernel(const F6
         for (int t = 0; t < ntiles; ++t) {
             const int b = t & 1;
             if (tid < PJT) {
-                tx[b][tid] = nx;
-                ty[b][tid] = ny;
-                tz[b][tid] = nz;
-                tm[b][tid] = nm;
-                th[b][tid] = nh;
+                T.x[b][tid] = nx;
+                T.y[b][tid] = ny;
+                T.z[b][tid] = nz;
+                T.m[b][tid] = nm;
+                T.h[b][tid] = nh;
             }
-            __syncthreads();  // the tile is staged; the last tile's reactions were read
+            // The tile is staged; the last tile's reactions were read.
+            const bool safe = !__syncthreads_or(!(safe_i && safe_body(nx, ny, nz, nh)));
             if (t + 1 < ntiles) fetch(t + 1);
             const int jt0 = w.j_begin + t * PJT;
             const bool sym = jt0 >= w.diag_end;
-#pragma unroll 1
-            for (int c0 = 0; c0 < PJT; c0 += 32) {
-                double r[NC];
+            const double2 cj = a.tile_class[jt0 / PJT];
+            const bool uni = uni_i && safe && cj.y > 0.0;
+            const double scale = uni ? cj.x : 1.0;
+            if (scale != scale_i || (t > 0 && (t & 7) == 0)) {
+                flush();
+                scale_i = scale;
+            }
+            if (uni) {
+                const double none[PK] = {};
+                const double H = ci.y + cj.y;
+                if (sym)
+                    fp64_pair_tile<ACC, PHI, true, true, true>(T, b, H, jw[warp], xi, yi, zi, none, none, ai, lane);
+                else
+                    fp64_pair_tile<ACC, PHI, false, true, true>(T, b, H, jw[warp], xi, yi, zi, none, none, ai, lane);
+            } else {
+                double hi[PK], mi[PK];
 #pragma unroll
-                for (int c = 0; c < NC; ++c) r[c] = 0.0;
-#pragma unroll kF64PUnroll
-                for (int s = 0; s < 32; ++s) {
-                    const int j = c0 + ((lane + s) & 31);
-                    const double xj = tx[b][j], yj = ty[b][j], zj = tz[b][j], mj = tm[b][j], hj = th[b][j];
-#pragma unroll
-                    for (int k = 0; k < PK; ++k) {
-                        const double dx = xj - xi[k], dy = yj - yi[k], dz = zj - zi[k];
-                        double r2 = hi[k] + hj;
-                        r2 = fma(dx, dx, r2);
-                        r2 = fma(dy, dy, r2);
-                        r2 = fma(dz, dz, r2);
-                        const double inv = rsqrt(r2);
-                        if (ACC) {
-                            const double i3 = inv * inv * inv;
-                            const double fi = mj * i3;
-                            ai[0][k] = fma(dx, fi, ai[0][k]);
-                            ai[1][k] = fma(dy, fi, ai[1][k]);
-                            ai[2][k] = fma(dz, fi, ai[2][k]);
-                            if (sym) {
-                                const double fj = mi[k] * i3;
-                                r[0] = fma(dx, fj, r[0]);
-                                r[1] = fma(dy, fj, r[1]);
-                                r[2] = fma(dz, fj, r[2]);
-                            }
-                        }
-                        if (PHI) {
-                            ai[CP][k] = fma(mj, inv, ai[CP][k]);
-                            if (sym) r[CP] = fma(mi[k], inv, r[CP]);
-                        }
-                    }
-                    if (sym) {
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) r[c] = __shfl_sync(0xffffffffu, r[c], src);
-                    }
+                for (int k = 0; k < PK; ++k) {
+                    const int64_t i = w.i_begin + k * PNT + tid;
+                    hi[k] = i < w.i_end ? 0.5 * a.eps2[i] : 1.0;
+                    mi[k] = i < w.i_end ? a.mass[i] : 0.0;
                 }
-                if (sym) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) jw[warp][c][c0 + lane] = r[c];
-                }
+                if (safe)
+                    if (sym) fp64_pair_tile<ACC, PHI, true, false, true>(T, b, 0.0, jw[warp], xi, yi, zi, hi, mi, ai, lane);
+                    else fp64_pair_tile<ACC, PHI, false, false, true>(T, b, 0.0, jw[warp], xi, yi, zi, hi, mi, ai, lane);
+                else if (sym)
+                    fp64_pair_tile<ACC, PHI, true, false, false>(T, b, 0.0, jw[warp], xi, yi, zi, hi, mi, ai, lane);
+                else
+                    fp64_pair_tile<ACC, PHI, false, false, false>(T, b, 0.0, jw[warp], xi, yi, zi, hi, mi, ai, lane);
             }
             if (sym) {
                 __syncthreads();  // every warp's reactions of the tile are in jw
@@ -270,32 +414,24 @@ __global__ void __launch_bounds__(PNT, KHRR_F64P_CTAS) fp64_pair_kernel(const F6
                             double v = 0.0;
 #pragma unroll
                             for (int q = 0; q < PW; ++q) v += jw[q][c][tid];
-                            s4[c] = v;
+                            s4[c] = uni ? ci.x * v : v;
                         }
                         // The reaction on j is minus the sum of m_i d / r^3
                         // (d = x_j - x_i); the potential's sum keeps its sign.
+                        const FxScale sc = a.scale[jt0 / PJT];
+                        double* u = a.sums + j;
                         if (ACC) {
-                            atomicAdd(&a.sums[j].x, -s4[0]);
-                            atomicAdd(&a.sums[j].y, -s4[1]);
-                            atomicAdd(&a.sums[j].z, -s4[2]);
+                            const double c = kCutGrid * sc.inv_acc;
+                            add_cut(u, lower, -s4[0], c);
+                            add_cut(u + a.npad, lower, -s4[1], c);
+                            add_cut(u + 2 * a.npad, lower, -s4[2], c);
                         }
-                        if (PHI) atomicAdd(&a.sums[j].w, s4[CP]);
+                        if (PHI) add_cut(u + 3 * a.npad, lower, s4[CP], kCutGrid * sc.inv_phi);
                     }
                 }
             }
         }
-#pragma unroll
-        for (int k = 0; k < PK; ++k) {
-            const int64_t i = w.i_begin + k * PNT + tid;
-            if (i < w.i_end && i < w.real_end) {
-                if (ACC) {
-                    atomicAdd(&a.sums[i].x, ai[0][k]);
-                    atomicAdd(&a.sums[i].y, ai[1][k]);
-                    atomicAdd(&a.sums[i].z, ai[2][k]);
-                }
-                if (PHI) atomicAdd(&a.sums[i].w, ai[CP][k]);
-            }
-        }
+        flush();
         // Every thread is done with the item (and s_item) before the next pull.
         __syncthreads();
     }

@@ -116,6 +116,12 @@ __device__ __forceinline__ void sum_partials(const StepArgs& a, int64_t i, d3& s
         sp = static_cast<double>(static_cast<long long>(a.fx[3 * a.npad + i])) * sc.inv_phi;
         return;
     }
+    if (a.f64) {
+        const double *u = a.f64 + i, *l = u + 4 * a.npad;
+        s = d3{u[0] + l[0], u[a.npad] + l[a.npad], u[2 * a.npad] + l[2 * a.npad]};
+        sp = u[3 * a.npad] + l[3 * a.npad];
+        return;
+    }
     const int ns = a.nsplit[i];
     for (int k = 0; k < ns; ++k) {
         const double4 p = a.part[k * a.npad + i];

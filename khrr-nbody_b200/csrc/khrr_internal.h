@@ -187,16 +187,19 @@ struct F64Args {
 };
 cudaError_t launch_fp64_force(const F64Args& a, bool acc, bool phi, int grid, cudaStream_t s);
 int fp64_force_ctas(int sm_count);  // resident CTAs of the FP64 kernel on the device
-// The symmetric FP64 pass on the pair kernel's plan: sums (ax, ay, az,
-// sum m/r per body, zeroed before the launch) accumulated with FP64 atomics.
+// The symmetric FP64 pass on plan_pair_tiles: sums (ax, ay, az, sum m/r per
+// body in two parts, zeroed before the launch) accumulated with FP64 atomics.
 struct F64PairArgs {
     const double* pos;      // AoS double3 [npad]
     const double* mass;     // [npad]
     const double* eps2;     // [npad]
-    const PairItem* items;  // plan_pair_items over 1024-body blocks
+    const PairItem* items;  // plan_pair_tiles
     int n_items;
     unsigned* queue;        // next-item counter (zeroed before each launch)
-    double4* sums;          // [npad]
+    double* sums;           // [2][4][npad]: upper and lower parts of ax, ay, az, sum m/r
+    long long npad;
+    const FxScale* scale;   // per 128-body tile (its powers of two set the cut)
+    const double2* tile_class;  // per 128-body tile: {mass, eps2 / 2}, {0, -1} for a mixed one
 };
 cudaError_t launch_fp64_pair(const F64PairArgs& a, bool acc, bool phi, int grid, cudaStream_t s);
 int fp64_pair_ctas(int sm_count);
@@ -217,6 +220,7 @@ struct StepArgs {
     const unsigned char* nsplit;  // partial slots per body
     const unsigned long long* fx;   // the pair kernel's fixed-point sums [kFxComps][npad] (replace part when set)
     const FxScale* fx_scale;        // their scales per 128-body tile
+    const double* f64;    // the symmetric FP64 pass's sums [2][4][npad] (replace part when set)
     int64_t n;            // padded count
     double dt;
     FieldConsts field;

@@ -87,6 +87,10 @@ PairBlocks pair_blocks_by_mass(const std::vector<int64_t>& poff, const std::vect
 // chosen from the CTA count), costliest first.
 void plan_pair_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int ctas, int chunk,
                      ForcePlan& out);
+// The same pairs cut at 128-body tiles (1024-body i blocks): chunks taper from
+// a quarter of a CTA's share of the work down to one tile, so layouts of any
+// size fill the persistent grid and its last round.
+void plan_pair_tiles(const std::vector<int64_t>& poff, const std::vector<int64_t>& cnt, int ctas, ForcePlan& out);
 
 // Force paths of the state API: the batched FP32 kernels (pair or one-sided,
 // per the tuning), the plain one-launch-per-system FP32 baseline (KHRR_PLAIN)
@@ -143,12 +147,14 @@ struct khrr_ctx {
     khrr::DevBuf<unsigned long long> fx;  // the pair kernel's fixed-point sums, kFxComps x npad
     khrr::DevBuf<khrr::FxScale> fx_scale; // their scale per 128-body tile
     std::vector<khrr::FxScale> fx_scales; // host copy (kept alive until the upload's copies complete)
+    khrr::DevBuf<double> f64_sums;  // the symmetric FP64 pass's sums, 2 x 4 x npad
     khrr::DevBuf<unsigned> queue, errflag;
     khrr::DevBuf<double> cons_blocks, scratch;
     bool uniform = false;
     float h_uniform = 0.0f;
     bool tile_uniform_mass = false;     // every 128-body tile of the layout has one mass
     khrr::DevBuf<float> tile_mass;      // that mass per tile (FP32)
+    khrr::DevBuf<double2> tile_class64; // per tile {mass, eps2 / 2} of a tile of 128 real bodies that share both, else {0, -1}
     bool block_uniform_mass = false;    // every pair block has one mass (the pair kernel's block-mass form)
     khrr::PairBlocks pair_blocks;       // the pair kernel's blocks of the layout
     khrr::FieldConsts field{};
