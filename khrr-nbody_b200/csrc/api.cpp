@@ -175,7 +175,7 @@ namespace khrr {
 // several, a split per system that brings every item near a common cost, the
 // items then run longest first.
 void plan_force_items(const std::vector<int64_t>& poff, const std::vector<int64_t>& cnt, int itile,
-                      int jt, int ctas, int forced_split, bool plain, ForcePlan& out) {
+                      int jt, int ctas, int sms, int forced_split, bool plain, ForcePlan& out) {
     out.items.clear();
     out.sys_item_begin.assign(cnt.size() + 1, 0);
     out.sys_split.assign(cnt.size(), 1);
@@ -197,6 +197,28 @@ void plan_force_items(const std::vector<int64_t>& poff, const std::vector<int64_
             s = 1;
         } else if (forced_split > 0) {
             s = std::min(forced_split, tiles);
+        } else if (nsys == 1 && 2 * nit * std::max(1, tiles / 8) < ctas) {
+            // Too few bodies for chunks of eight tiles to fill half the grid:
+            // the split with the least estimated time.  An SM's share is its
+            // items times the tiles of one (a CTA alone on an SM reaches 80 %
+            // of the SM's rate), and every chunk's partial sums are written and
+            // read back.  Measured on the packed 128 x 4 shape: 3.7 us per
+            // 128-body tile and SM, ~1 us per item, 64 bytes per slot and body
+            // at 5 TB/s.  Per pass (events around the call, us): 1,000 bodies
+            // 53 -> 15, 3,072 45 -> 15 (144 items instead of 18), 6,144 47 ->
+            // 27, 10,007 95 -> 67; from 14,336 bodies on the rule below is better
+            // (101 against 102; 30,000: 414 against 443).
+            const double tile_us = 3.7 * itile / 512.0;
+            double best = 1e300;
+            for (int c = 1; c <= std::min(64, tiles); ++c) {
+                const double per_sm = std::ceil(static_cast<double>(nit) * c / std::max(sms, 1));
+                const double item = tile_us * std::ceil(static_cast<double>(tiles) / c) + 1.0;
+                const double t = item * (per_sm > 1.0 ? per_sm : 1.25) + 1.3e-5 * c * static_cast<double>(np);
+                if (t < 0.995 * best) {
+                    best = t;
+                    s = c;
+                }
+            }
         } else if (nsys == 1) {
             // Best last-wave fill; chunks of at least 8 tiles; ties -> fewer chunks.
             double best = -1.0;
@@ -375,7 +397,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
                            "upload items")) != KHRR_OK)
                 return st;
         } else {
-            plan_force_items(poff, cnt, kF64ITile, kPad, ctas, 0, false, p);
+            plan_force_items(poff, cnt, kF64ITile, kPad, ctas, sm_count, 0, false, p);
             if ((st = cuda(p.d_items.ensure(p.items.size()), "alloc items")) != KHRR_OK) return st;
             if ((st = cuda(cudaMemcpyAsync(p.d_items.p, p.items.data(), p.items.size() * sizeof(WorkItem),
                                            cudaMemcpyHostToDevice, stream),
@@ -435,7 +457,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
     if (p.valid && !p.pair && p.threads == v->threads && p.ipt == v->i_per_thread && p.jt == v->j_tile &&
         p.split_req == tuning.j_split && p.ctas == ctas)
         return KHRR_OK;
-    plan_force_items(poff, cnt, v->threads * v->i_per_thread, v->j_tile, ctas, tuning.j_split, plain, p);
+    plan_force_items(poff, cnt, v->threads * v->i_per_thread, v->j_tile, ctas, sm_count, tuning.j_split, plain, p);
     p.pair = false;
     p.threads = v->threads;
     p.ipt = v->i_per_thread;

@@ -114,7 +114,7 @@ khrr_status prepare_kernel_pass(khrr_ctx* c, const double* pos_i, const double* 
     if (!p.valid || p.pair || c->kplan_n != n || p.threads != v->threads || p.ipt != v->i_per_thread ||
         p.split_req != c->tuning.j_split || p.ctas != ctas) {
         std::vector<int64_t> poff{0, npad}, cnt{n};
-        plan_force_items(poff, cnt, v->threads * v->i_per_thread, v->j_tile, ctas, c->tuning.j_split, false, p);
+        plan_force_items(poff, cnt, v->threads * v->i_per_thread, v->j_tile, ctas, c->sm_count, c->tuning.j_split, false, p);
         p.pair = false;
         p.threads = v->threads;
         p.ipt = v->i_per_thread;

@@ -74,7 +74,7 @@ struct ForcePlan {
 };
 
 void plan_force_items(const std::vector<int64_t>& poff, const std::vector<int64_t>& cnt, int itile,
-                      int jt, int ctas, int forced_split, bool plain, ForcePlan& out);
+                      int jt, int ctas, int sms, int forced_split, bool plain, ForcePlan& out);
 // The symmetric pair kernel's blocks: per system the padded indices
 // P_k = b_0 < b_1 < ... < b_nb = P_{k+1}, each block at most kPairBlock
 // bodies starting at a multiple of kPad.
