@@ -425,6 +425,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
         }
         if ((st = cuda(cudaStreamSynchronize(stream), "plan sync")) != KHRR_OK) return st;
         p.valid = true;
+        clean = 0;
         drop_graphs();  // captured graphs may hold the old queue or partial buffer
         return KHRR_OK;
     }
@@ -451,6 +452,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
             return st;
         if ((st = cuda(cudaStreamSynchronize(stream), "plan sync")) != KHRR_OK) return st;
         p.valid = true;
+        clean = 0;
         drop_graphs();
         return KHRR_OK;
     }
@@ -482,6 +484,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
         return st;
     if ((st = cuda(cudaStreamSynchronize(stream), "plan sync")) != KHRR_OK) return st;
     p.valid = true;
+    clean = 0;
     drop_graphs();
     return KHRR_OK;
 }
@@ -518,6 +521,21 @@ ForceArgs khrr_ctx::force_args(const ForcePlan& p, int item_begin, int item_end)
     return a;
 }
 
+khrr_status khrr_ctx::ensure_clean(int mode) {
+    if (mode == kModePlain) return KHRR_OK;  // no queue, no accumulated sums
+    const ForcePlan& p = plan_for(mode);
+    const int kind = p.pair ? kCleanFx : (p.f64_pair ? kCleanF64 : kCleanQueue);
+    if (clean == kind) return KHRR_OK;
+    clean = 0;
+    khrr_status st = cuda(cudaMemsetAsync(queue.p, 0, sizeof(unsigned), stream), "queue reset");
+    if (st == KHRR_OK && kind == kCleanFx)
+        st = cuda(cudaMemsetAsync(fx.p, 0, sizeof(unsigned long long) * kFxComps * npad, stream), "sums reset");
+    if (st == KHRR_OK && kind == kCleanF64)
+        st = cuda(cudaMemsetAsync(f64_sums.p, 0, 8 * sizeof(double) * npad, stream), "sums reset");
+    if (st == KHRR_OK) clean = kind;
+    return st;
+}
+
 khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, const double* x) {
     const bool plain = mode == kModePlain;
     const ForceVariant* v = variant(uniform, acc, phi);
@@ -531,9 +549,6 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
     if (events && (st = cuda(cudaEventRecordWithFlags(ph0, stream, cudaEventRecordExternal), "event")) != KHRR_OK)
         return st;
     if (mode == kModeF64 && p.f64_pair) {
-        if ((st = cuda(cudaMemsetAsync(queue.p, 0, sizeof(unsigned), stream), "queue reset")) != KHRR_OK) return st;
-        if ((st = cuda(cudaMemsetAsync(f64_sums.p, 0, 8 * sizeof(double) * npad, stream), "sums reset")) != KHRR_OK)
-            return st;
         F64PairArgs a{};
         a.pos = x;
         a.mass = mass.p;
@@ -549,7 +564,6 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
             KHRR_OK)
             return st;
     } else if (mode == kModeF64) {
-        if ((st = cuda(cudaMemsetAsync(queue.p, 0, sizeof(unsigned), stream), "queue reset")) != KHRR_OK) return st;
         F64Args a{};
         a.pos = x;
         a.mass = mass.p;
@@ -579,10 +593,6 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
         }
     } else if (p.pair) {
         if (!v->pair) return fail(KHRR_ERR_INVALID_ARG, "no pair kernel for this output set");
-        if ((st = cuda(cudaMemsetAsync(queue.p, 0, sizeof(unsigned), stream), "queue reset")) != KHRR_OK) return st;
-        if ((st = cuda(cudaMemsetAsync(fx.p, 0, sizeof(unsigned long long) * kFxComps * npad, stream),
-                       "sums reset")) != KHRR_OK)
-            return st;
         PairArgs a{};
         a.sh = shadow();
         a.items = p.d_pair_items.p;
@@ -597,7 +607,6 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
         if ((st = cuda(launch_pair(v, a, std::min(a.n_items, ctas), stream), "pair force kernel")) != KHRR_OK)
             return st;
     } else {
-        if ((st = cuda(cudaMemsetAsync(queue.p, 0, sizeof(unsigned), stream), "queue reset")) != KHRR_OK) return st;
         const int e = static_cast<int>(p.items.size());
         if ((st = cuda(launch_force(v, force_args(p, 0, e), std::min(e, ctas), stream), "force kernel")) != KHRR_OK)
             return st;
@@ -623,6 +632,7 @@ StepArgs khrr_ctx::step_args(const ForcePlan& p, double dt) {
     a.nsplit = p.d_nsplit.p;
     a.fx = p.pair ? fx.p : nullptr;
     a.f64 = p.f64_pair ? f64_sums.p : nullptr;
+    a.queue = queue.p;
     a.fx_scale = fx_scale.p;
     a.n = npad;
     a.dt = dt;
@@ -630,9 +640,9 @@ StepArgs khrr_ctx::step_args(const ForcePlan& p, double dt) {
     return a;
 }
 
-khrr_status khrr_ctx::enqueue_step(double dt, int mode, bool phi_now, bool compat) {
+khrr_status khrr_ctx::enqueue_step(double dt, int mode, bool phi_now, bool compat, bool events) {
     const bool plain = mode == kModePlain;
-    khrr_status st = enqueue_force(mode, true, phi_now, true, post.p);
+    khrr_status st = enqueue_force(mode, true, phi_now, events, post.p);
     if (st != KHRR_OK) return st;
     ForcePlan& p = plan_for(mode);
     StepArgs sa = step_args(p, dt);
@@ -641,6 +651,7 @@ khrr_status khrr_ctx::enqueue_step(double dt, int mode, bool phi_now, bool compa
     sa.predict_next = 1;
     if (!plain) return cuda(launch_corrector(sa, stream), "corrector");
     // Baseline path: one launch per system for the integrator as well.
+    sa.queue = nullptr;
     for (size_t k = 0; k < cnt.size(); ++k) {
         StepArgs s = sa;
         const int64_t o = poff[k];
@@ -672,7 +683,7 @@ khrr_status khrr_ctx::get_step_graph(double dt, int mode, bool phi_now, bool com
     if (st != KHRR_OK) return st;
     uint64_t dt_bits;
     std::memcpy(&dt_bits, &dt, sizeof dt_bits);
-    const auto key = std::make_tuple(dt_bits, mode, phi_now, compat);
+    const auto key = std::make_tuple(dt_bits, mode, phi_now, compat, timing);
     auto it = graphs.find(key);
     if (it != graphs.end()) {
         *out = &it->second;
@@ -681,7 +692,7 @@ khrr_status khrr_ctx::get_step_graph(double dt, int mode, bool phi_now, bool com
     StepGraph g{};
     if ((st = cuda(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture")) != KHRR_OK)
         return st;
-    khrr_status est = enqueue_step(dt, mode, phi_now, compat);
+    khrr_status est = enqueue_step(dt, mode, phi_now, compat, timing);
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(stream, &graph);
     if (est != KHRR_OK) {
@@ -794,6 +805,7 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
     if (cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ph0) != cudaSuccess || cudaEventCreate(&c->ph1) != cudaSuccess ||
         c->queue.ensure(1) != cudaSuccess || c->errflag.ensure(1) != cudaSuccess ||
+        c->cons_done.ensure(1) != cudaSuccess ||
         c->scratch.ensure(64) != cudaSuccess) {
         khrr_destroy(c);
         return KHRR_ERR_CUDA;
@@ -801,6 +813,7 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
     c->stream = c->own;
     cudaMemset(c->queue.p, 0, sizeof(unsigned));
     cudaMemset(c->errflag.p, 0, sizeof(unsigned));
+    cudaMemset(c->cons_done.p, 0, sizeof(unsigned));
     for (int i = 0; i < force_variant_count() + pair_variant_count(); ++i) {
         const ForceVariant* v = i < force_variant_count() ? force_variant(i) : pair_variant(i - force_variant_count());
         if (cudaFuncSetAttribute(v->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -904,6 +917,7 @@ khrr_status khrr_upload_state(khrr_ctx* c, int64_t n, const double* pos, const d
     // state.
     c->has_state = false;
     c->predicted = false;
+    c->clean = 0;
     c->off = off;
     c->cnt = cnt;
     c->poff = poff;
@@ -1113,6 +1127,8 @@ khrr_status khrr_forces(khrr_ctx* c, int flags) {
     const bool plain = mode == kModePlain;
     cudaStream_t s = c->stream;
     khrr_status st;
+    if ((st = c->ensure_plan(mode)) != KHRR_OK || (st = c->ensure_clean(mode)) != KHRR_OK) return st;
+    c->clean = 0;  // until the collect below is on its way
     // Shadow of the current positions (a previous step leaves the predicted ones).
     if ((st = c->cuda(launch_pack(c->pos.p, c->mass.p, c->eps2.p, c->npad, c->npad, c->shadow(), s),
                       "pack")) != KHRR_OK)
@@ -1131,6 +1147,7 @@ khrr_status khrr_forces(khrr_ctx* c, int flags) {
     sa.want_phi = want_phi ? 1 : 0;
     if ((st = c->cuda(launch_collect(sa, want_acc, (flags & KHRR_COMPAT_ACCUMULATE) != 0, s), "collect")) != KHRR_OK)
         return st;
+    c->clean = plain ? 0 : (p.pair ? khrr_ctx::kCleanFx : (p.f64_pair ? khrr_ctx::kCleanF64 : khrr_ctx::kCleanQueue));
     c->predicted = false;
     return KHRR_OK;
 }
@@ -1157,13 +1174,19 @@ khrr_status khrr_step(khrr_ctx* c, double dt, int nsteps, int flags) {
         const bool phi_now = phi_last && k == nsteps - 1;
         StepGraph* g = nullptr;
         if ((st = c->get_step_graph(dt, mode, phi_now, compat, &g)) != KHRR_OK) return st;
-        if (!g->ev0 || !g->ev1) return c->fail(KHRR_ERR_CUDA, "step graph lacks its timing event nodes");
-        cudaEvent_t e0 = c->ph0, e1 = c->ph1;
-        if (c->timing && (st = c->timing_pair(&e0, &e1)) != KHRR_OK) return st;
-        if ((st = c->cuda(cudaGraphExecEventRecordNodeSetEvent(g->exec, g->ev0, e0), "graph event")) != KHRR_OK ||
-            (st = c->cuda(cudaGraphExecEventRecordNodeSetEvent(g->exec, g->ev1, e1), "graph event")) != KHRR_OK)
+        if (c->timing) {
+            if (!g->ev0 || !g->ev1) return c->fail(KHRR_ERR_CUDA, "step graph lacks its timing event nodes");
+            cudaEvent_t e0 = nullptr, e1 = nullptr;
+            if ((st = c->timing_pair(&e0, &e1)) != KHRR_OK ||
+                (st = c->cuda(cudaGraphExecEventRecordNodeSetEvent(g->exec, g->ev0, e0), "graph event")) != KHRR_OK ||
+                (st = c->cuda(cudaGraphExecEventRecordNodeSetEvent(g->exec, g->ev1, e1), "graph event")) != KHRR_OK)
+                return st;
+        }
+        if ((st = c->ensure_clean(mode)) != KHRR_OK) return st;
+        if ((st = c->cuda(cudaGraphLaunch(g->exec, s), "graph launch")) != KHRR_OK) {
+            c->clean = 0;
             return st;
-        if ((st = c->cuda(cudaGraphLaunch(g->exec, s), "graph launch")) != KHRR_OK) return st;
+        }
         if (c->timing) {
             c->timed_launches += plain ? static_cast<int64_t>(c->cnt.size()) : 1;
             c->timed_pairs += c->pairs_per_pass();
@@ -1182,7 +1205,7 @@ khrr_status khrr_conservation(khrr_ctx* c, khrr_lie* out) {
     khrr_status st;
     if ((st = c->cuda(c->cons_blocks.ensure(static_cast<size_t>(nb) * 16), "alloc")) != KHRR_OK) return st;
     if ((st = c->cuda(launch_conservation(c->pos.p, c->vel.p, c->mass.p, c->phi.p, c->npad, c->cons_blocks.p,
-                                          nb, c->scratch.p, c->stream),
+                                          nb, c->cons_done.p, c->scratch.p, c->stream),
                       "conservation")) != KHRR_OK)
         return st;
     double v[16];

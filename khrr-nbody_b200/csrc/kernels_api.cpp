@@ -147,6 +147,7 @@ khrr_status prepare_kernel_pass(khrr_ctx* c, const double* pos_i, const double* 
 
 khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i) {
     ForcePlan& p = c->kplan;
+    c->clean = 0;  // the state's force passes share the queue counter
     const int64_t npad = round_up(c->kplan_n, kPad);
     if (v->pair) {
         PairArgs a{};

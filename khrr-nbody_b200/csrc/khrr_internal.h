@@ -218,9 +218,10 @@ struct StepArgs {
     const double4* part;  // force partials [slot][npad]
     long long npad;
     const unsigned char* nsplit;  // partial slots per body
-    const unsigned long long* fx;   // the pair kernel's fixed-point sums [kFxComps][npad] (replace part when set)
+    unsigned long long* fx;         // the pair kernel's fixed-point sums [kFxComps][npad] (replace part when set)
     const FxScale* fx_scale;        // their scales per 128-body tile
-    const double* f64;    // the symmetric FP64 pass's sums [2][4][npad] (replace part when set)
+    double* f64;          // the symmetric FP64 pass's sums [2][4][npad] (replace part when set)
+    unsigned* queue;      // zeroed for the next force pass (when set), as fx and f64 are after they were read
     int64_t n;            // padded count
     double dt;
     FieldConsts field;
@@ -236,10 +237,11 @@ cudaError_t launch_collect(const StepArgs& a, bool want_acc, bool accumulate, cu
 cudaError_t launch_integ_time(const double* acc, double* pos_t, double* vel_t, const double* pos,
                               const double* vel, double dt, int istep, double* acc0, int64_t n,
                               const FieldConsts& f, cudaStream_t s);
-// FP64 conservation sums over bodies (ghosts have zero mass and contribute
+// FP64 conservation sums over bodies; done: a word that is zero before the
+// call and after it (ghosts have zero mass and contribute
 // nothing to the sums; they sit at the origin with zero velocity).
 cudaError_t launch_conservation(const double* pos, const double* vel, const double* mass,
-                                const double* phi, int64_t n, double* block_out, int nblocks,
+                                const double* phi, int64_t n, double* block_out, int nblocks, unsigned* done,
                                 double* out16, cudaStream_t s);
 int conservation_blocks(int64_t n);
 

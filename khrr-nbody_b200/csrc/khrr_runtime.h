@@ -150,6 +150,7 @@ struct khrr_ctx {
     khrr::DevBuf<double> f64_sums;  // the symmetric FP64 pass's sums, 2 x 4 x npad
     khrr::DevBuf<unsigned> queue, errflag;
     khrr::DevBuf<double> cons_blocks, scratch;
+    khrr::DevBuf<unsigned> cons_done;  // khrr_conservation's count of finished blocks (zero between calls)
     bool uniform = false;
     float h_uniform = 0.0f;
     bool tile_uniform_mass = false;     // every 128-body tile of the layout has one mass
@@ -162,7 +163,13 @@ struct khrr_ctx {
     khrr::ForcePlan plan_batched, plan_plain, plan_fp64;
     bool predicted = false;
     double pred_dt = 0.0;
-    std::map<std::tuple<uint64_t, int, bool, bool>, khrr::StepGraph> graphs;  // (dt, mode, phi, compat)
+    std::map<std::tuple<uint64_t, int, bool, bool, bool>, khrr::StepGraph> graphs;  // (dt, mode, phi, compat, timed)
+    // Every force pass starts from a zero queue counter and, where its kernel
+    // accumulates, zero sums; the kernel that reads the sums zeroes both again.
+    // clean: the kind of pass they are zero for (0: unknown).
+    enum { kCleanQueue = 1, kCleanFx = 2, kCleanF64 = 3 };
+    int clean = 0;
+    khrr_status ensure_clean(int mode);
 
     // Kernel-level entry points: their own shadow, partials and plan.
     khrr::DevBuf<float> kshadow, kishadow;
@@ -226,7 +233,7 @@ struct khrr_ctx {
     khrr_status enqueue_force(int mode, bool acc, bool phi, bool events, const double* x);
     khrr::StepArgs step_args(const khrr::ForcePlan& p, double dt);
     khrr::Shadow shadow() { return khrr::shadow_at(shadow_buf.p, npad); }
-    khrr_status enqueue_step(double dt, int mode, bool phi_now, bool compat);
+    khrr_status enqueue_step(double dt, int mode, bool phi_now, bool compat, bool events);
     khrr_status get_step_graph(double dt, int mode, bool phi_now, bool compat, khrr::StepGraph** out);
     khrr_status timing_pair(cudaEvent_t* e0, cudaEvent_t* e1);
     khrr_status call_start();  // with timing on: event before the call's first kernel
