@@ -337,6 +337,20 @@ void plan_pair_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, 
                      [](const PairItem& a, const PairItem& b) { return a.cost > b.cost; });
 }
 
+// A CTA takes as long for a short i block as for a full one, so the time goes
+// with the j tiles (the i block's own tiles: 11 packed operations against 14).
+void weigh_pair_items(int sms, ForcePlan& out) {
+    uint64_t total = 0;
+    for (PairItem& it : out.pair_items) {
+        const int own = std::max(0, std::min(it.diag_end, it.j_end) - it.j_begin) / kPad;
+        it.weight = 5 * ((it.j_end - it.j_begin) / kPad) - own;
+        total += static_cast<uint64_t>(it.weight);
+    }
+    std::stable_sort(out.pair_items.begin(), out.pair_items.end(),
+                     [](const PairItem& a, const PairItem& b) { return a.weight > b.weight; });
+    out.pair_share = static_cast<unsigned>(std::min<uint64_t>((total + sms - 1) / sms, 0xffffffffu));
+}
+
 // Work in units of one i block against one j tile.  A chunk's size at any
 // point is a quarter of what is left divided by the CTAs (at most 256 tiles,
 // at least one): few items while much is left, single tiles at the end, so
@@ -437,6 +451,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
     if (!plain && v->pair) {
         if (p.valid && p.pair && p.split_req == tuning.j_split && p.ctas == ctas) return KHRR_OK;
         plan_pair_items(pair_blocks, cnt, ctas, tuning.j_split, p);
+        weigh_pair_items(sm_count, p);
         p.pair = true;
         p.threads = v->threads;
         p.ipt = v->i_per_thread;
@@ -527,7 +542,7 @@ khrr_status khrr_ctx::ensure_clean(int mode) {
     const int kind = p.pair ? kCleanFx : (p.f64_pair ? kCleanF64 : kCleanQueue);
     if (clean == kind) return KHRR_OK;
     clean = 0;
-    khrr_status st = cuda(cudaMemsetAsync(queue.p, 0, sizeof(unsigned), stream), "queue reset");
+    khrr_status st = cuda(cudaMemsetAsync(queue.p, 0, kQueueWords * sizeof(unsigned), stream), "queue reset");
     if (st == KHRR_OK && kind == kCleanFx)
         st = cuda(cudaMemsetAsync(fx.p, 0, sizeof(unsigned long long) * kFxComps * npad, stream), "sums reset");
     if (st == KHRR_OK && kind == kCleanF64)
@@ -598,6 +613,7 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
         a.items = p.d_pair_items.p;
         a.n_items = static_cast<int>(p.pair_items.size());
         a.queue = queue.p;
+        a.share = p.pair_share;
         a.fx = fx.p;
         a.npad = npad;
         a.scale = fx_scale.p;
@@ -804,14 +820,14 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
     c->sm_count = prop.multiProcessorCount;
     if (cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ph0) != cudaSuccess || cudaEventCreate(&c->ph1) != cudaSuccess ||
-        c->queue.ensure(1) != cudaSuccess || c->errflag.ensure(1) != cudaSuccess ||
+        c->queue.ensure(kQueueWords) != cudaSuccess || c->errflag.ensure(1) != cudaSuccess ||
         c->cons_done.ensure(1) != cudaSuccess ||
         c->scratch.ensure(64) != cudaSuccess) {
         khrr_destroy(c);
         return KHRR_ERR_CUDA;
     }
     c->stream = c->own;
-    cudaMemset(c->queue.p, 0, sizeof(unsigned));
+    cudaMemset(c->queue.p, 0, kQueueWords * sizeof(unsigned));
     cudaMemset(c->errflag.p, 0, sizeof(unsigned));
     cudaMemset(c->cons_done.p, 0, sizeof(unsigned));
     for (int i = 0; i < force_variant_count() + pair_variant_count(); ++i) {

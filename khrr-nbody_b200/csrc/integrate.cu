@@ -110,7 +110,8 @@ __global__ void predictor_kernel(const StepArgs a) {
 __device__ __forceinline__ void sum_partials(const StepArgs& a, int64_t i, d3& s, double& sp) {
     s = d3{0.0, 0.0, 0.0};
     sp = 0.0;
-    if (a.queue && i == 0) *a.queue = 0u;
+    if (a.queue)
+        for (int64_t q = i; q < kQueueWords; q += a.n) a.queue[q] = 0u;
     if (a.fx) {
         // The pair kernel's fixed-point sums (zero for ghosts).
         const FxScale sc = a.fx_scale[i / kPad];

@@ -61,6 +61,7 @@ khrr_status prepare_pair_pass(khrr_ctx* c, const double* mass, const double* eps
     if (!p.valid || !p.pair || c->kplan_n != n || p.split_req != c->tuning.j_split || p.ctas != ctas) {
         std::vector<int64_t> cnt{n};
         plan_pair_items(pair_blocks_fixed({0, npad}), cnt, ctas, c->tuning.j_split, p);
+        weigh_pair_items(c->sm_count, p);
         p.pair = true;
         p.threads = v->threads;
         p.ipt = v->i_per_thread;
@@ -155,6 +156,7 @@ khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i)
         a.items = p.d_pair_items.p;
         a.n_items = static_cast<int>(p.pair_items.size());
         a.queue = c->queue.p;
+        a.share = p.pair_share;
         a.fx = c->kfx.p;
         a.npad = npad;
         a.scale = c->kscale.p;
@@ -165,7 +167,7 @@ khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i)
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         khrr_status st;
         if (c->timing && (st = c->timing_pair(&e0, &e1)) != KHRR_OK) return st;
-        if ((st = c->cuda(cudaMemsetAsync(c->queue.p, 0, sizeof(unsigned), s), "queue reset")) != KHRR_OK) return st;
+        if ((st = c->cuda(cudaMemsetAsync(c->queue.p, 0, kQueueWords * sizeof(unsigned), s), "queue reset")) != KHRR_OK) return st;
         if ((st = c->cuda(cudaMemsetAsync(c->kfx.p, 0, sizeof(unsigned long long) * kFxComps * npad, s),
                           "sums reset")) != KHRR_OK)
             return st;

@@ -87,8 +87,11 @@ struct PairItem {
     int diag_end;  // == j_begin when the chunk holds no tile of the i block
     int real_end;  // end of the system's real bodies
     int cost;      // planner's estimate (i bodies x j bodies / 1024)
-    int pad;
+    int weight;    // its time: 5 per tile, 4 per tile of the i block
 };
+// Words of the force queue: the next-item counter; for the pair kernel also
+// the CTAs that stopped at their SM's share and the weight each SM has taken.
+constexpr int kQueueStopped = 1, kQueueLoad = 2, kQueueSms = 256, kQueueWords = kQueueLoad + kQueueSms;
 
 // The pair kernel's results are 64-bit fixed-point sums: every partial (an
 // FP32 sum) is scaled by a power of two and rounded to an integer, then added
@@ -113,7 +116,8 @@ struct PairArgs {
     Shadow sh;               // the bodies (i and j are the same set)
     const PairItem* items;
     int n_items;
-    unsigned* queue;         // next-item counter (zeroed before each launch)
+    unsigned* queue;         // kQueueWords words (zeroed before each launch)
+    unsigned share;          // an SM's share of the items' weight
     unsigned long long* fx;  // fixed-point sums [kFxComps][npad] (zeroed before each launch)
     long long npad;          // component stride
     const FxScale* scale;    // per 128-body tile

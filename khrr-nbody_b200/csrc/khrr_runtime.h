@@ -67,6 +67,7 @@ struct ForcePlan {
     bool pair = false;
     bool f64_pair = false;  // FP64 plan: the symmetric FP64 kernel on pair_items
     std::vector<PairItem> pair_items;
+    unsigned pair_share = 0;  // an SM's share of the items' weight
     DevBuf<PairItem> d_pair_items;
     ForcePlan() = default;
     ForcePlan(const ForcePlan&) = delete;
@@ -85,6 +86,9 @@ PairBlocks pair_blocks_fixed(const std::vector<int64_t>& poff);
 PairBlocks pair_blocks_by_mass(const std::vector<int64_t>& poff, const std::vector<float>& tile_mass);
 // The pair kernel's items: block rows cut into chunks of `chunk` blocks (0 =
 // chosen from the CTA count), costliest first.
+// Time weights of a pair plan's items, heaviest first, and the share of one of
+// `sms` SMs.
+void weigh_pair_items(int sms, ForcePlan& out);
 void plan_pair_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int ctas, int chunk,
                      ForcePlan& out);
 // The same pairs cut at 128-body tiles (1024-body i blocks): chunks taper from

@@ -41,7 +41,11 @@
 // item): d (3 add), r^2 (3 fma), two MUFU.RSQ, r^-3 (2 mul), i side (3 fma),
 // j side (3 fma) = 14 f32x2 instructions per two pair evaluations, that is 14
 // FP32 operations per evaluation of an unordered pair and 7 per interaction,
-// against 11 per interaction for the one-sided kernel.  When every block has one
+// against 11 per interaction for the one-sided kernel.  (What holds the pass
+// at 35.7 cycles per two pairs and scheduler instead of the 28 in which the 14
+// would issue: a packed FMA of three different operands takes 3.05 cycles to
+// read its registers, one of two 2.05-2.25, measured on plain chains, so the
+// six sums' FMAs cost 18 of 34.)  When every block has one
 // mass (and no ghosts) the masses are factored out of both sums; otherwise
 // m_j and m_i enter per pair (2 more multiplies).
 //
@@ -99,11 +103,11 @@ static_assert(NT * K == kPairBlock, "block = threads x bodies per thread");
 static_assert(JT == NT, "one thread per j body writes the reaction partials");
 static_assert(JT % 64 == 0 && JT == kPad, "tiles are whole sub-chunk pairs and padding units");
 
-// Unroll of the 32-step loop, measured at 786k bodies: 2 for accelerations
-// (149.6 ms per pass against 153.1 for 1 and 151.2 for 4), 1 with the
-// potential (168.9 ms against 171.1 for 2 and 175.4 for 4).
+// Unroll of the 32-step loop, ms per pass at 786k bodies: accelerations 147.5
+// for 1 (16.40 at 262k), 148.5 for 2 (16.55), 151.2 for 4; with the potential
+// 168.9 for 1, 171.1 for 2, 175.4 for 4.
 #ifndef KHRR_PAIR_UNROLL
-#define KHRR_PAIR_UNROLL 2
+#define KHRR_PAIR_UNROLL 1
 #endif
 constexpr int kSUnroll = KHRR_PAIR_UNROLL;
 // Tiles per fold of the acceleration-only variants' i-side partials,
@@ -180,15 +184,13 @@ __device__ __forceinline__ void pair_tile(const float* __restrict__ tile, float*
                 if (ACC) {
                     const float2 i3 = __fmul2_rn(inv, __fmul2_rn(inv, inv));
                     const float2 fi = BMASS ? i3 : __fmul2_rn(M2, i3);
+                    const float2 fj = BMASS ? i3 : __fmul2_rn(mi[k], i3);
                     ai[0][k] = __ffma2_rn(dx, fi, ai[0][k]);
+                    if (SYM) rx = __ffma2_rn(dx, fj, rx);
                     ai[1][k] = __ffma2_rn(dy, fi, ai[1][k]);
+                    if (SYM) ry = __ffma2_rn(dy, fj, ry);
                     ai[2][k] = __ffma2_rn(dz, fi, ai[2][k]);
-                    if (SYM) {
-                        const float2 fj = BMASS ? i3 : __fmul2_rn(mi[k], i3);
-                        rx = __ffma2_rn(dx, fj, rx);
-                        ry = __ffma2_rn(dy, fj, ry);
-                        rz = __ffma2_rn(dz, fj, rz);
-                    }
+                    if (SYM) rz = __ffma2_rn(dz, fj, rz);
                 }
                 if (PHI) {
                     ai[CP][k] = BMASS ? __fadd2_rn(ai[CP][k], inv) : __ffma2_rn(M2, inv, ai[CP][k]);
@@ -238,6 +240,25 @@ constexpr int pair_min_blocks() {
     return ((F & kAcc) && (F & kPhi) && !((F & kUnif) && (F & kBMass))) ? 2 : 3;
 }
 
+// The CTA's next item (>= n_items: none).  An SM's CTAs share its FP32
+// datapath, so with a few items per SM the pass ends when the SM with the
+// most items does, and CTAs that pull freely finish in step: the SMs whose
+// three come first take three more items each and the others none (1,176
+// items at 49,152 bodies: nine on most SMs where eight on each would do).  So
+// an SM stops pulling once it has taken its share of the weight; the last CTA
+// of the grid never stops, whatever the shares and wherever the CTAs run.
+// Per acceleration pass 684 -> 627 us at 49,152 bodies, 327 -> 307 at 30,720,
+// 4302 -> 4213 at 131,072; from 786k on (0.1 %) it makes no difference.
+__device__ __forceinline__ int next_item(const PairArgs& a) {
+    unsigned sm;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    const unsigned ahead = *reinterpret_cast<volatile unsigned*>(a.queue);
+    if (ahead >= static_cast<unsigned>(a.n_items)) return a.n_items;
+    const unsigned taken = atomicAdd(a.queue + kQueueLoad + sm % kQueueSms, static_cast<unsigned>(a.items[ahead].weight));
+    if (taken >= a.share && atomicAdd(a.queue + kQueueStopped, 1u) + 1u < gridDim.x) return a.n_items;
+    return static_cast<int>(atomicAdd(a.queue, 1u));
+}
+
 template <unsigned F>
 __global__ void __launch_bounds__(NT, (pair_min_blocks<F>())) pair_kernel(const PairArgs a) {
     using S = PairShape<F>;
@@ -276,7 +297,7 @@ __global__ void __launch_bounds__(NT, (pair_min_blocks<F>())) pair_kernel(const 
     const float2 e2 = f2(a.h_uniform + a.h_uniform, a.h_uniform + a.h_uniform);
     unsigned consumed = 0;  // tiles this CTA has consumed, over all its items
     for (;;) {
-        if (tid == 0) s_item = static_cast<int>(atomicAdd(a.queue, 1u));
+        if (tid == 0) s_item = next_item(a);
         __syncthreads();
         const int it = s_item;
         if (it >= a.n_items) break;
