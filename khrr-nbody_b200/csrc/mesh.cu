@@ -29,32 +29,16 @@
 #include "async_copy.cuh"
 #include "khrr_internal.h"
 #include "wave_bricks.h"
+#include "wave_march.cuh"
 
 namespace khrr {
 namespace {
-
-constexpr double kPi = 3.14159265358979;  // the reference's PI (common.cuh:7)
 
 int grid_for(int64_t n, int block) {
     int64_t g = (n + block - 1) / block;
     if (g > 148 * 32) g = 148 * 32;
     if (g < 1) g = 1;
     return static_cast<int>(g);
-}
-
-// a / b, correctly rounded, from y = RN(1/b): Markstein's correction step
-// (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Develop. 34(1), 1990; see also
-// Muller et al., "Handbook of Floating-Point Arithmetic", ch. 4): q = RN(a y)
-// is within an ulp of a/b, r = a - b q is exact in one fma, and RN(q + r y)
-// is RN(a/b).  Several quotients over one denominator then share one
-// correctly rounded reciprocal (__drcp_rn).  Checked bitwise against the IEEE
-// division on 1.7e10 quotients (the stencil's operand ranges and random
-// operands over 64 binary orders of magnitude): no difference.
-__device__ __forceinline__ double div_rn(double a, double b, double y) {
-    const double q = __dmul_rn(a, y);
-    const double r = fma(-b, q, a);
-    return fma(r, y, q);
 }
 
 // Cell coordinate of one axis: (int)((p - lo) / cs) clamped to [0, g - 1],
@@ -352,106 +336,12 @@ __device__ __forceinline__ int64_t at3(int x, int y, int z, int nx) {
     return static_cast<int64_t>(x) + static_cast<int64_t>(y) * nx + static_cast<int64_t>(z) * nx * nx;
 }
 
-// Sponge of wave-kernel.cuh:32-60 (coordinates ix*dx, not centred; the x
-// test compares against -(L - bc)).
-__device__ __forceinline__ double wave_diss(const WaveConsts& W, int ix, int iy, int iz) {
-    const double x = ix * W.dx, y = iy * W.dx, z = iz * W.dx;
-    const double L = W.sim_l - W.bc_l;
-    double d = W.diss_base;
-    if (x > -L) d += W.diss_extra * fabs(x - L) * fabs(x - L);
-    else if (x < -L) d += W.diss_extra * fabs(x + L) * fabs(x + L);
-    if (y > L) d += W.diss_extra * fabs(y - L) * fabs(y - L);
-    else if (y < -L) d += W.diss_extra * fabs(y + L) * fabs(y + L);
-    if (z > L) d += W.diss_extra * fabs(z - L) * fabs(z - L);
-    else if (z < -L) d += W.diss_extra * fabs(z + L) * fabs(z + L);
-    return d;
-}
-
-
-// wave_diss_iteration in FP64, the reference's expressions term for term
-// (same bits as the literal per-cell kernel): kWZ consecutive z cells of one
-// (x, y) column per thread with every load issued up front, K computed once
-// per thread, and the five per-cell divisions (rho and the four coefficients
-// over Wt) through shared correctly rounded reciprocals: 1.41x the literal
-// kernel at 256^3.
-template <int kWZ>
-__global__ void __launch_bounds__(256) wave_f64_kernel(double* __restrict__ phi_new, const double* __restrict__ phi,
-                                                       const double* __restrict__ phi_old,
-                                                       const double* __restrict__ mass, const WaveConsts W) {
-    const int NX = W.nx;
-    const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y;
-    const int zb = blockIdx.z * kWZ;
-    if (ix >= NX || iy >= NX) return;
-    const int64_t sy = NX, sz = static_cast<int64_t>(NX) * NX;
-    const int64_t col = static_cast<int64_t>(iy) * NX + ix;
-    const int64_t dxm = ix > 0 ? 1 : 0, dxp = ix < NX - 1 ? 1 : 0;
-    const int64_t dym = iy > 0 ? sy : 0, dyp = iy < NX - 1 ? sy : 0;
-    double c[kWZ + 2];
-    double xm[kWZ], xp[kWZ], ym[kWZ], yp[kWZ], po[kWZ], ms[kWZ];
-#pragma unroll
-    for (int u = 0; u < kWZ + 2; ++u) c[u] = phi[min(max(zb - 1 + u, 0), NX - 1) * sz + col];
-#pragma unroll
-    for (int u = 0; u < kWZ; ++u) {
-        const int64_t at = min(zb + u, NX - 1) * sz + col;
-        xm[u] = phi[at - dxm];
-        xp[u] = phi[at + dxp];
-        ym[u] = phi[at - dym];
-        yp[u] = phi[at + dyp];
-        po[u] = phi_old[at];
-        ms[u] = mass[at];
-    }
-    const bool edge_xy = ix == 0 || ix == NX - 1 || iy == 0 || iy == NX - 1;
-    const double DX = W.dx, C = W.c, DT = W.dt;
-    const double D3 = DX * DX * DX;
-    const double yD3 = __drcp_rn(D3);
-    const double K = C * C * (DT * DT) / (DX * DX);
-    const double KFn = -(C * C) * (DT * DT);
-    const double KAn = 2 * (1. - 3 * K);
-#pragma unroll
-    for (int u = 0; u < kWZ; ++u) {
-        const int z = zb + u;
-        if (z >= NX) break;
-        double out = 0.0;
-        if (!(edge_xy || z == 0 || z == NX - 1)) {
-            const double rho = div_rn(ms[u], D3, yD3);
-            const double f = 4 * kPi * 1.0 * rho;
-            const double diss = wave_diss(W, ix, iy, z);
-            const double Q = diss * C * DT * 0.5;
-            const double Wt = 1 + Q;
-            const double yW = __drcp_rn(Wt);
-            const double KM = div_rn(K, Wt, yW);
-            const double KF = div_rn(KFn, Wt, yW);
-            const double KA = div_rn(KAn, Wt, yW);
-            const double KO = div_rn(Q - 1., Wt, yW);
-            out = xm[u] * KM + xp[u] * KM + ym[u] * KM + yp[u] * KM + c[u] * KM + c[u + 2] * KM + c[u + 1] * KA +
-                  po[u] * KO + f * KF;
-        }
-        phi_new[z * sz + col] = out;
-    }
-}
-
-// The FP32 form of the step.  The sponge is separable,
-// diss = base + sx[ix] + sy[iy] + sz[iz] (per-axis tables built in FP64 on the
-// host); per cell: Q = diss c dt / 2, w = 1 / (1 + Q), and
-//   phi_new = nb K w + phi (2 (1 - 3K)) w + phi_old (Q - 1) w + mass S w,
-// with nb the six-neighbour sum and S = -c^2 dt^2 4 pi / dx^3.  With resid,
-// sum (phi_new - phi)^2 and sum phi_new^2 are accumulated in FP64.
-// Each thread computes kWZ consecutive z cells of one (x, y) column: the
-// column's phi values are loaded once and shared as z neighbours, and all
-// other loads (x/y neighbours, phi_old, mass) are issued up front, so a warp
-// keeps many requests in flight (no barriers, no shared memory).  kWZ = 8 on
-// large meshes, 4 on small ones (more CTAs).
-// CTA shape in x (a multiple of 32: each warp is one x row segment) and y.
-#ifndef KHRR_WAVE_WX
-#define KHRR_WAVE_WX 32
-#endif
-#ifndef KHRR_WAVE_WY
-#define KHRR_WAVE_WY 8
-#endif
-constexpr int kWX = KHRR_WAVE_WX, kWY = KHRR_WAVE_WY;
-
-
-static_assert(kWX % 32 == 0 && kWX * kWY <= 1024, "whole warps along x");
+// The FP32 step where the rows are not whole 16-byte packs (nx % 4 != 0):
+// each thread computes kWZ consecutive z cells of one (x, y) column, all loads
+// issued up front, so 4-byte loads keep as many bytes in flight (201^3: 38.0
+// us per iteration; the march of wave_march.cuh with single cells 51.7).
+// kWZ = 8 on large meshes, 4 on small ones (more CTAs).
+constexpr int kWX = 32, kWY = 8;  // threads in x (one warp per row segment) and y
 
 template <int kWZ>
 __global__ void __launch_bounds__(kWX * kWY) wave_f32_kernel(float* __restrict__ phi_new, const float* __restrict__ phi,
@@ -522,107 +412,6 @@ __global__ void __launch_bounds__(kWX * kWY) wave_f32_kernel(float* __restrict__
             n2 += __shfl_xor_sync(0xffffffffu, n2, o);
         }
         if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&resid[0], d2);
-            atomicAdd(&resid[1], n2);
-        }
-    }
-}
-
-// The same step with four consecutive x cells per thread (nx % 4 == 0):
-// every row access is one 16-byte load or store, so a warp moves 512
-// contiguous bytes per access and issues a quarter of the load instructions.
-// The x neighbours come from the float4 itself and, across threads, by warp
-// shuffles (a warp covers 128 consecutive x cells); lanes 0 and 31 load the
-// one cell beyond their warp's span.  Threads past the mesh in x read
-// clamped addresses (for the shuffles) and store nothing.  Per cell the
-// arithmetic is wave_f32_kernel's, so the bits are the same.
-constexpr int kW4X = 32, kW4Y = 8;  // threads: 128 x cells x 8 rows
-
-__device__ __forceinline__ float f4c(const float4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
-
-template <int kWZ>
-__global__ void __launch_bounds__(kW4X * kW4Y) wave_f32x4_kernel(float* __restrict__ phi_new, const float* __restrict__ phi,
-                                                                 const float* __restrict__ phi_old,
-                                                                 const float* __restrict__ mass, const WaveF32 W,
-                                                                 double* __restrict__ resid) {
-    const int NX = W.nx;
-    const int ix0 = (blockIdx.x * kW4X + threadIdx.x) * 4, iy = blockIdx.y * kW4Y + threadIdx.y;
-    const int zb = blockIdx.z * kWZ;
-    const int lane = threadIdx.x;  // kW4X == 32: one warp per x row segment
-    const int64_t sy = NX, sz = static_cast<int64_t>(NX) * NX;
-    double d2 = 0.0, n2 = 0.0;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (iy < NX) {  // whole warps share iy: the shuffles below see every lane
-        const bool xin = ix0 < NX;
-        const int xc = xin ? ix0 : NX - 4;  // clamped for the loads
-        const int64_t col = static_cast<int64_t>(iy) * NX + xc;
-        const int64_t dym = iy > 0 ? sy : 0, dyp = iy < NX - 1 ? sy : 0;
-        const int64_t dxm = xc > 0 ? 1 : 0, dxp = xc + 4 < NX ? 4 : 3;  // the cells beyond the float4
-        float4 c[kWZ + 2];  // phi at z = zb - 1 .. zb + kWZ (clamped)
-        float4 ym[kWZ], yp[kWZ], po[kWZ], ms[kWZ];
-        float xl[kWZ], xr[kWZ];  // lanes 0 / 31: phi at xc - 1 / xc + 4
-#pragma unroll
-        for (int u = 0; u < kWZ + 2; ++u) {
-            const int z = min(max(zb - 1 + u, 0), NX - 1);
-            c[u] = *reinterpret_cast<const float4*>(phi + z * sz + col);
-        }
-#pragma unroll
-        for (int u = 0; u < kWZ; ++u) {
-            const int64_t at = min(zb + u, NX - 1) * sz + col;
-            ym[u] = *reinterpret_cast<const float4*>(phi + at - dym);
-            yp[u] = *reinterpret_cast<const float4*>(phi + at + dyp);
-            po[u] = *reinterpret_cast<const float4*>(phi_old + at);
-            ms[u] = *reinterpret_cast<const float4*>(mass + at);
-            xl[u] = lane == 0 ? phi[at - dxm] : 0.0f;
-            xr[u] = lane == 31 ? phi[at + dxp] : 0.0f;
-        }
-        const float4 sx4 = *reinterpret_cast<const float4*>(W.sx + xc);
-        const float sy1 = W.sy[iy];
-        const bool edge_y = iy == 0 || iy == NX - 1;
-#pragma unroll
-        for (int u = 0; u < kWZ; ++u) {
-            const int z = zb + u;
-            const float4 cc = c[u + 1];
-            // x neighbours of the end cells from the adjacent lanes
-            float left = __shfl_up_sync(0xffffffffu, cc.w, 1);
-            float right = __shfl_down_sync(0xffffffffu, cc.x, 1);
-            if (lane == 0) left = xl[u];
-            if (lane == 31) right = xr[u];
-            if (z >= NX || !xin) continue;
-            const int64_t at = z * sz + col;
-            float out[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int ix = xc + k;
-                float o = 0.0f;
-                if (!(edge_y || ix == 0 || ix == NX - 1 || z == 0 || z == NX - 1)) {
-                    const float xm = k == 0 ? left : f4c(cc, k - 1);
-                    const float xp = k == 3 ? right : f4c(cc, k + 1);
-                    const float nb = ((xm + xp) + (f4c(ym[u], k) + f4c(yp[u], k))) + (f4c(c[u], k) + f4c(c[u + 2], k));
-                    const float diss = ((W.diss_base + f4c(sx4, k)) + sy1) + W.sz[z];
-                    const float Q = diss * W.cdt_half;
-                    const float w = __frcp_rn(1.0f + Q);  // correctly rounded: the bits of 1.0f / (1.0f + Q)
-                    o = fmaf(nb, W.K * w,
-                             fmaf(f4c(cc, k), W.A * w, fmaf(f4c(po[u], k), (Q - 1.0f) * w, f4c(ms[u], k) * (W.S * w))));
-                }
-                out[k] = o;
-                if (resid) {
-                    const double dd = static_cast<double>(o) - static_cast<double>(f4c(cc, k));
-                    d2 += dd * dd;
-                    n2 += static_cast<double>(o) * static_cast<double>(o);
-                }
-            }
-            *reinterpret_cast<float4*>(phi_new + at) = make_float4(out[0], out[1], out[2], out[3]);
-        }
-    }
-    if (resid) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            d2 += __shfl_xor_sync(0xffffffffu, d2, o);
-            n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-        }
-        if (lane == 0) {
             atomicAdd(&resid[0], d2);
             atomicAdd(&resid[1], n2);
         }
@@ -1471,19 +1260,29 @@ cudaError_t launch_cell_phi(const double* phi, const int2* pci, const int* count
 
 cudaError_t launch_wave_f64(double* phi_new, const double* phi, const double* phi_old, const double* mass,
                             const WaveConsts& w, cudaStream_t s) {
-    // One cell per thread: the FP64 update is bound by its FP64 arithmetic,
-    // so occupancy (48 registers) beats more cells per thread (measured at
-    // 256^3: 151.7 us per iteration against 155.9 for 2 and 169.3 for 4).
-    const dim3 block(32, 8), grid((w.nx + 31) / 32, (w.nx + 7) / 8, w.nx);
-    wave_f64_kernel<1><<<grid, block, 0, s>>>(phi_new, phi, phi_old, mass, w);
-    return cudaGetLastError();
+    // Pairs of cells where the rows and the caller's arrays allow 16-byte
+    // accesses.  us per iteration at 64^3 / 100^3 / 128^3 / 200^3 / 256^3: 3.2 /
+    // 6.8 / 12.2 / 54.7 / 108.9 (one cell per thread and launch of 249
+    // instructions a cell: 6.2 / 14.5 / 20.6 / 82.5 / 153.5); 128 threads, five
+    // blocks per SM; 256 x 2 2.8 / 7.1 / 12.0 / 60.6 / 120.3, six blocks spill
+    // (75.7 at 200^3).  Single cells (201^3): 64.6 against 84.5.
+    const uintptr_t any = reinterpret_cast<uintptr_t>(phi_new) | reinterpret_cast<uintptr_t>(phi) |
+                          reinterpret_cast<uintptr_t>(phi_old) | reinterpret_cast<uintptr_t>(mass);
+    if (w.nx % 2 == 0 && any % 16 == 0)
+        return launch_march<StepF64<2>, 2, 128, 5, false>(phi_new, phi, phi_old, mass, w, w.nx, nullptr, s);
+    return launch_march<StepF64<1>, 1, 256, 4, false>(phi_new, phi, phi_old, mass, w, w.nx, nullptr, s);
 }
 
 cudaError_t launch_wave_f32(float* phi_new, const float* phi, const float* phi_old, const float* mass,
                             const WaveF32& w, double* resid, cudaStream_t s) {
-    // Launched with programmatic stream serialization: a chain of steps
-    // overlaps each grid's launch with the previous grid's tail (measured
-    // ~2 % on the 507-step Wave-mode chain at 128^3; same bits).
+    // 16-byte packs where the rows allow them (the solvers' arrays are
+    // aligned).  us per iteration at 64^3 / 100^3 / 160^3 / 200^3 / 256^3: 2.6 /
+    // 4.5 / 11.2 / 24.8 / 51.7 (5.2 TB/s of 16 bytes a cell) with 256 threads
+    // and three blocks per SM; 4.0 / 6.2 / 20.4 / 36.9 / 68.4 before; four
+    // blocks (64 registers) spill: 68.3 at 256^3.
+    if (w.nx % 4 == 0)
+        return resid ? launch_march<StepF32<4>, 4, 256, 3, true>(phi_new, phi, phi_old, mass, w, w.nx, resid, s)
+                     : launch_march<StepF32<4>, 4, 256, 3, false>(phi_new, phi, phi_old, mass, w, w.nx, resid, s);
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kWX, kWY);
     cfg.stream = s;
@@ -1492,20 +1291,10 @@ cudaError_t launch_wave_f32(float* phi_new, const float* phi, const float* phi_o
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    // Kernel choice, measured (us per iteration, 128^3 / 256^3): one cell per
-    // thread with 4 / 8 z planes 12.5 / 71.8; four x cells per thread with 2 z
-    // planes 12.0 / 72.3 (with 4 planes 12.8 / 79.6).
-    if (w.nx < 192 && w.nx % 4 == 0 && w.nx >= 8) {
-        cfg.blockDim = dim3(kW4X, kW4Y);
-        cfg.gridDim = dim3((w.nx + 4 * kW4X - 1) / (4 * kW4X), (w.nx + kW4Y - 1) / kW4Y, (w.nx + 1) / 2);
-        return cudaLaunchKernelEx(&cfg, wave_f32x4_kernel<2>, phi_new, phi, phi_old, mass, w, resid);
-    }
-    if (w.nx >= 192) {
-        cfg.gridDim = dim3((w.nx + kWX - 1) / kWX, (w.nx + kWY - 1) / kWY, (w.nx + 7) / 8);
-        return cudaLaunchKernelEx(&cfg, wave_f32_kernel<8>, phi_new, phi, phi_old, mass, w, resid);
-    }
-    cfg.gridDim = dim3((w.nx + kWX - 1) / kWX, (w.nx + kWY - 1) / kWY, (w.nx + 3) / 4);
-    return cudaLaunchKernelEx(&cfg, wave_f32_kernel<4>, phi_new, phi, phi_old, mass, w, resid);
+    const int per = w.nx >= 192 ? 8 : 4;
+    cfg.gridDim = dim3((w.nx + kWX - 1) / kWX, (w.nx + kWY - 1) / kWY, (w.nx + per - 1) / per);
+    return cudaLaunchKernelEx(&cfg, per == 8 ? wave_f32_kernel<8> : wave_f32_kernel<4>, phi_new, phi, phi_old, mass, w,
+                              resid);
 }
 
 bool wave_resident_available(int nx) {
