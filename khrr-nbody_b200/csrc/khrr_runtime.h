@@ -115,6 +115,8 @@ struct MeshSolver {
     MeshGeom geom{};
     int64_t cells = 0;
     DevBuf<double> cell_mass, phi64, cell_acc;  // C, 4 C (field ring), 3 C
+    DevBuf<double> copies;                      // cic_copy_count meshes: zero between deposits
+    int ncopies = 0;
     DevBuf<float> mass32, phi32, tab;           // C, 4 C (field ring), 3 nx
     DevBuf<int2> pci;                           // npad
     DevBuf<double4> part;                       // npad: {acc, -phi} per body
@@ -195,6 +197,8 @@ struct khrr_ctx {
     khrr::DevBuf<int> mcount, mstart, maxpbc, mscan, mtmp;  // mscan: scan block/tile totals
     khrr::DevBuf<int> morder;                            // khrr_sort_by_cell: n body indices
     khrr::DevBuf<double> cell_mass, cell_phi, wave_resid;
+    khrr::DevBuf<double> cic_copies;                     // khrr_cic_deposit's extra meshes, zero between calls
+    bool cic_deposited = false;                          // a deposit was made without them
     int64_t cell_phi_cells = 0;                          // mesh size the cell_phi sums belong to
     khrr::DevBuf<float> wave_phi, wave_mass, wave_tab;   // 4 C (field ring), C, 3 nx
     int wave_nx = 0;

@@ -1084,14 +1084,31 @@ __device__ __forceinline__ CicAxis cic_axis(double p, double lo, double cs, doub
     return a;
 }
 
-__global__ void cic_deposit_kernel(const double* __restrict__ pos, const double* __restrict__ mass, int64_t n,
-                                   const MeshGeom m, double* __restrict__ cell_mass) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// Two neighbouring lanes share a body, one per x corner: the two cells of a
+// row are neighbours in memory, so a warp's access touches 16-20 lines instead
+// of 32, and the deposit's two reductions meet in one sector at L2.  Measured
+// against one lane per body (us; 786,432 bodies): deposit 113.7 -> 82.1 on the
+// two-galaxy encounter at 128^3 (the rest is reductions on the same cells of
+// the dense cores: 32.8 -> 20.9 for uniform bodies), 418 -> 304 for one galaxy
+// at 32^3; 168 -> 111 for 2.1 M bodies at 256^3.  Eight lanes per body, a
+// corner each and the axes shared by shuffles, execute more instructions than
+// that saves (147, and 138 for the gather).
+__global__ void __launch_bounds__(256) cic_deposit_kernel(const double* __restrict__ pos,
+                                                          const double* __restrict__ mass, int64_t n, const MeshGeom m,
+                                                          double* __restrict__ cell_mass, double* __restrict__ copies,
+                                                          int ncopies, int64_t cells) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, i = t >> 1;
     if (i >= n) return;
+    const int a = static_cast<int>(t & 1);
+    const int own = static_cast<int>(blockIdx.x % static_cast<unsigned>(ncopies + 1));
+    double* const out = own == 0 ? cell_mass : copies + (own - 1) * cells;
     const CicAxis ax = cic_axis(pos[3 * i], m.lo[0], m.cs[0], m.rcs[0], m.g[0]);
     const CicAxis ay = cic_axis(pos[3 * i + 1], m.lo[1], m.cs[1], m.rcs[1], m.g[1]);
     const CicAxis az = cic_axis(pos[3 * i + 2], m.lo[2], m.cs[2], m.rcs[2], m.g[2]);
     const double mi = mass[i];
+    const int x = ax.i0 + a;
+    if (x < 0 || x >= m.g[0]) return;
+    const double wx = a ? ax.w[1] : ax.w[0];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int z = az.i0 + c;
@@ -1100,61 +1117,82 @@ __global__ void cic_deposit_kernel(const double* __restrict__ pos, const double*
         for (int b = 0; b < 2; ++b) {
             const int y = ay.i0 + b;
             if (y < 0 || y >= m.g[1]) continue;
-#pragma unroll
-            for (int a = 0; a < 2; ++a) {
-                const int x = ax.i0 + a;
-                if (x < 0 || x >= m.g[0]) continue;
-                const double w = (ax.w[a] * ay.w[b]) * az.w[c];
-                atomicAdd(&cell_mass[static_cast<int64_t>(z) * m.g[0] * m.g[1] + static_cast<int64_t>(y) * m.g[2] + x],
-                          mi * w);
-            }
+            const double w = (wx * ay.w[b]) * az.w[c];
+            atomicAdd(&out[static_cast<int64_t>(z) * m.g[0] * m.g[1] + static_cast<int64_t>(y) * m.g[2] + x], mi * w);
         }
     }
 }
 
-// Interpolation back to a body: acc (3 per cell) and a scalar field in FP32
-// or FP64; sums in z, y, x corner order.
+// The copies' sums into the cells, the copies zero again.
+__global__ void __launch_bounds__(256) cic_combine_kernel(double* __restrict__ cell_mass, double* __restrict__ copies,
+                                                          int ncopies, int64_t cells) {
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= cells) return;
+    double s = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < ncopies; ++k) s += copies[k * cells + c];
+    cell_mass[c] += s;
+#pragma unroll 4
+    for (int k = 0; k < ncopies; ++k) copies[k * cells + c] = 0.0;
+}
+
+// Interpolation back to a body by its two lanes (a: the lane's x corner): acc
+// (3 per cell) and a scalar field in FP32 or FP64.  The products of the second
+// corner reach the first lane by shuffle and the sums run in z, y, x corner
+// order there, as one thread would form them; corners outside the mesh add
+// nothing.  Every lane of the warp takes part (p: any address in bounds for
+// lanes past the bodies).  The result is the first lane's.
 template <class T>
-__device__ __forceinline__ void cic_interp(const double* __restrict__ p, const MeshGeom& m,
+__device__ __forceinline__ void cic_interp(const double* __restrict__ p, int a, const MeshGeom& m,
                                            const double* __restrict__ cacc, const T* __restrict__ cval, double (&acc)[3],
                                            double& val) {
     const CicAxis ax = cic_axis(p[0], m.lo[0], m.cs[0], m.rcs[0], m.g[0]);
     const CicAxis ay = cic_axis(p[1], m.lo[1], m.cs[1], m.rcs[1], m.g[1]);
     const CicAxis az = cic_axis(p[2], m.lo[2], m.cs[2], m.rcs[2], m.g[2]);
+    const int x = ax.i0 + a;
+    const bool x_in = x >= 0 && x < m.g[0];
+    const bool x0_in = ax.i0 >= 0 && ax.i0 < m.g[0], x1_in = ax.i0 + 1 >= 0 && ax.i0 + 1 < m.g[0];
+    const double wx = a ? ax.w[1] : ax.w[0];
     acc[0] = acc[1] = acc[2] = 0.0;
     val = 0.0;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int z = az.i0 + c;
-        if (z < 0 || z >= m.g[2]) continue;
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const int y = ay.i0 + b;
-            if (y < 0 || y >= m.g[1]) continue;
-#pragma unroll
-            for (int a = 0; a < 2; ++a) {
-                const int x = ax.i0 + a;
-                if (x < 0 || x >= m.g[0]) continue;
-                const double w = (ax.w[a] * ay.w[b]) * az.w[c];
+            const bool row_in = z >= 0 && z < m.g[2] && y >= 0 && y < m.g[1];
+            double q[4] = {0.0, 0.0, 0.0, 0.0};
+            if (row_in && x_in) {
+                const double w = (wx * ay.w[b]) * az.w[c];
                 const int64_t id = static_cast<int64_t>(z) * m.g[0] * m.g[1] + static_cast<int64_t>(y) * m.g[2] + x;
                 if (cacc) {
-                    acc[0] += w * cacc[3 * id];
-                    acc[1] += w * cacc[3 * id + 1];
-                    acc[2] += w * cacc[3 * id + 2];
+                    q[0] = w * cacc[3 * id];
+                    q[1] = w * cacc[3 * id + 1];
+                    q[2] = w * cacc[3 * id + 2];
                 }
-                if (cval) val += w * static_cast<double>(cval[id]);
+                if (cval) q[3] = w * static_cast<double>(cval[id]);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (k < 3 ? !cacc : !cval) continue;
+                const double second = __shfl_down_sync(0xffffffffu, q[k], 1);
+                double& sum = k < 3 ? acc[k] : val;
+                if (row_in && x0_in) sum += q[k];
+                if (row_in && x1_in) sum += second;
             }
         }
     }
 }
 
-__global__ void cic_gather_kernel(const double* __restrict__ pos, int64_t n, const MeshGeom m,
-                                  const double* __restrict__ cacc, const double* __restrict__ cval,
-                                  double* __restrict__ pacc, double* __restrict__ pval) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__global__ void __launch_bounds__(256) cic_gather_kernel(const double* __restrict__ pos, int64_t n, const MeshGeom m,
+                                                         const double* __restrict__ cacc,
+                                                         const double* __restrict__ cval, double* __restrict__ pacc,
+                                                         double* __restrict__ pval) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, i = t >> 1;
     double a[3], v;
-    cic_interp(pos + 3 * i, m, pacc ? cacc : nullptr, pval ? cval : nullptr, a, v);
+    cic_interp(pos + 3 * min(i, n - 1), static_cast<int>(t & 1), m, pacc ? cacc : nullptr, pval ? cval : nullptr, a, v);
+    if (i >= n || (t & 1)) return;
     if (pacc) {
         pacc[3 * i] = a[0];
         pacc[3 * i + 1] = a[1];
@@ -1166,23 +1204,23 @@ __global__ void cic_gather_kernel(const double* __restrict__ pos, int64_t n, con
 // The mesh-force gather into the corrector's partial slot: {acc, -phi}, so
 // the corrector's phi = 0 - (-phi) is the mesh potential (apply_acceleration_
 // to_particles and apply_cell_to_particles, p2mesh-kernel.cuh:227-254).
-template <bool CIC, class T>
-__global__ void mesh_gather_kernel(const double* __restrict__ pos, const int2* __restrict__ pci, int64_t n,
-                                   const MeshGeom m, const double* __restrict__ cacc, const T* __restrict__ phi,
-                                   double4* __restrict__ part) {
+template <class T>
+__global__ void __launch_bounds__(256) mesh_gather_cic_kernel(const double* __restrict__ pos, int64_t n,
+                                                              const MeshGeom m, const double* __restrict__ cacc,
+                                                              const T* __restrict__ phi, double4* __restrict__ part) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, i = t >> 1;
+    double a[3], v;
+    cic_interp(pos + 3 * min(i, n - 1), static_cast<int>(t & 1), m, cacc, phi, a, v);
+    if (i < n && !(t & 1)) part[i] = make_double4(a[0], a[1], a[2], -v);
+}
+
+template <class T>
+__global__ void mesh_gather_ngp_kernel(const int2* __restrict__ pci, int64_t n, const double* __restrict__ cacc,
+                                       const T* __restrict__ phi, double4* __restrict__ part) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double a[3], v;
-    if (CIC) {
-        cic_interp(pos + 3 * i, m, cacc, phi, a, v);
-    } else {
-        const int64_t c = pci[i].x;
-        a[0] = cacc[3 * c];
-        a[1] = cacc[3 * c + 1];
-        a[2] = cacc[3 * c + 2];
-        v = static_cast<double>(phi[c]);
-    }
-    part[i] = make_double4(a[0], a[1], a[2], -v);
+    const int64_t c = pci[i].x;
+    part[i] = make_double4(cacc[3 * c], cacc[3 * c + 1], cacc[3 * c + 2], -static_cast<double>(phi[c]));
 }
 
 // acc_field on an FP32 potential: the float differences are exact in FP64.
@@ -1423,18 +1461,37 @@ cudaError_t launch_deinterleave(const int2* pci, int64_t n, int* a, int* b, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_cic_deposit(const double* pos, const double* mass, int64_t n, const MeshGeom& m,
-                               double* cell_mass, cudaStream_t s) {
+// Extra meshes for the deposit: the dense cells' reductions land on the same
+// sectors one after another, 15 ns each (564 us for a 786,432-body galaxy on
+// 32^3 cells over [-4, 4]^3, where its uniform share would take 20), and with
+// R meshes R of them proceed at once.  Adding the copies up costs R cells of
+// reads and writes, so R goes with the bodies per cell and the meshes stay
+// within 69 MB.  Measured (us, one mesh -> with copies): 786,432 bodies 32^3
+// 564 -> 77, 64^3 209 -> 56, 96^3 146 -> 56, 128^3 68 -> 53; 2 M on 32^3 1428 ->
+// 180, on 160^3 211 -> 164; 20,000 on 32^3 23 -> 13, on 48^3 10 -> 15 (one mesh
+// kept).  Uniformly spread bodies pay for it: 23 -> 31 at 64^3, 21 -> 37 at
+// 128^3.
+int cic_copy_count(int64_t n, int64_t cells) {
+    const int64_t meshes = std::min<int64_t>({16, 8 * n / cells, int64_t(8600000) / cells});
+    return meshes < 2 ? 0 : static_cast<int>(meshes) - 1;
+}
+
+cudaError_t launch_cic_deposit(const double* pos, const double* mass, int64_t n, const MeshGeom& m, double* cell_mass,
+                               double* copies, int ncopies, cudaStream_t s) {
     if (n < 1) return cudaSuccess;
-    cic_deposit_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(pos, mass, n, m, cell_mass);
+    const int64_t cells = static_cast<int64_t>(m.g[0]) * m.g[1] * m.g[2];
+    cic_deposit_kernel<<<static_cast<unsigned>((2 * n + 255) / 256), 256, 0, s>>>(pos, mass, n, m, cell_mass, copies,
+                                                                                  ncopies, cells);
+    if (ncopies > 0)
+        cic_combine_kernel<<<static_cast<unsigned>((cells + 255) / 256), 256, 0, s>>>(cell_mass, copies, ncopies, cells);
     return cudaGetLastError();
 }
 
 cudaError_t launch_cic_gather(const double* pos, int64_t n, const MeshGeom& m, const double* cell_acc,
                               const double* cell_value, double* pacc, double* pval, cudaStream_t s) {
     if (n < 1) return cudaSuccess;
-    cic_gather_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(pos, n, m, cell_acc, cell_value, pacc,
-                                                                               pval);
+    cic_gather_kernel<<<static_cast<unsigned>((2 * n + 255) / 256), 256, 0, s>>>(pos, n, m, cell_acc, cell_value, pacc,
+                                                                                   pval);
     return cudaGetLastError();
 }
 
@@ -1448,13 +1505,14 @@ cudaError_t launch_mesh_gather(const double* pos, const int2* pci, int64_t n, co
                                const double* cell_acc, const float* phi32, const double* phi64, double4* part,
                                cudaStream_t s) {
     if (n < 1) return cudaSuccess;
-    const unsigned g = static_cast<unsigned>((n + 255) / 256);
     if (cic) {
-        if (phi32) mesh_gather_kernel<true, float><<<g, 256, 0, s>>>(pos, pci, n, m, cell_acc, phi32, part);
-        else mesh_gather_kernel<true, double><<<g, 256, 0, s>>>(pos, pci, n, m, cell_acc, phi64, part);
+        const unsigned g = static_cast<unsigned>((2 * n + 255) / 256);
+        if (phi32) mesh_gather_cic_kernel<float><<<g, 256, 0, s>>>(pos, n, m, cell_acc, phi32, part);
+        else mesh_gather_cic_kernel<double><<<g, 256, 0, s>>>(pos, n, m, cell_acc, phi64, part);
     } else {
-        if (phi32) mesh_gather_kernel<false, float><<<g, 256, 0, s>>>(pos, pci, n, m, cell_acc, phi32, part);
-        else mesh_gather_kernel<false, double><<<g, 256, 0, s>>>(pos, pci, n, m, cell_acc, phi64, part);
+        const unsigned g = static_cast<unsigned>((n + 255) / 256);
+        if (phi32) mesh_gather_ngp_kernel<float><<<g, 256, 0, s>>>(pci, n, cell_acc, phi32, part);
+        else mesh_gather_ngp_kernel<double><<<g, 256, 0, s>>>(pci, n, cell_acc, phi64, part);
     }
     return cudaGetLastError();
 }

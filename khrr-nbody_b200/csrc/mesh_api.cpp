@@ -489,7 +489,31 @@ khrr_status khrr_cic_deposit(khrr_ctx* c, const double* pos, const double* mass,
     khrr_status st = check_cubic(c, mesh, &g, &C);
     if (st != KHRR_OK) return st;
     if (n < 0 || (n > 0 && (!pos || !mass || !cell_mass))) return c->fail(KHRR_ERR_INVALID_ARG, "bad deposit arguments");
-    return c->cuda(launch_cic_deposit(pos, mass, n, g, cell_mass, c->stream), "cic deposit");
+    // The copies are the context's; a capture of the caller's keeps none of its
+    // pointers and deposits directly.
+    int copies = cic_copy_count(n, C);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (copies > 0 && (st = c->cuda(cudaStreamIsCapturing(c->stream, &capture), "capture status")) != KHRR_OK) return st;
+    if (capture != cudaStreamCaptureStatusNone) copies = 0;
+    if (copies > 0) {
+        const size_t need = static_cast<size_t>(copies) * static_cast<size_t>(C);
+        if (c->cic_copies.n < need && !c->cic_deposited) {
+            // Allocating them takes as long as some twenty deposits save: from
+            // the context's second deposit on.
+            c->cic_deposited = true;
+            copies = 0;
+        } else if (c->cic_copies.n < need) {
+            if (c->cic_copies.ensure(need) != cudaSuccess) {
+                (void)cudaGetLastError();  // no room: deposit directly
+                copies = 0;
+            } else if ((st = c->cuda(cudaMemsetAsync(c->cic_copies.p, 0, need * sizeof(double), c->stream), "memset")) !=
+                       KHRR_OK) {
+                c->cic_copies.release();
+                return st;
+            }
+        }
+    }
+    return c->cuda(launch_cic_deposit(pos, mass, n, g, cell_mass, c->cic_copies.p, copies, c->stream), "cic deposit");
 }
 
 khrr_status khrr_cic_gather(khrr_ctx* c, const double* pos, int64_t n, const khrr_mesh* mesh, const double* cell_acc,
@@ -605,9 +629,24 @@ khrr_status khrr_ctx::mesh_ensure_layout() {
     // All bodies share the one mesh: several independent systems would
     // attract each other through it.
     if (cnt.size() != 1) return fail(KHRR_ERR_INVALID_ARG, "the mesh solver runs one system (got %zu)", cnt.size());
+    khrr_status st;
+    const int want = M.cfg.assign == KHRR_ASSIGN_CIC ? cic_copy_count(cnt[0], M.cells) : 0;
+    const size_t need = static_cast<size_t>(want) * static_cast<size_t>(M.cells);
+    if (want != M.ncopies || need > M.copies.n) {
+        M.drop_graphs();
+        M.ncopies = 0;
+        if (need > M.copies.n) {
+            if (M.copies.ensure(need) != cudaSuccess) {
+                (void)cudaGetLastError();  // no room: deposit directly
+            } else if ((st = cuda(cudaMemsetAsync(M.copies.p, 0, need * sizeof(double), stream), "memset")) != KHRR_OK) {
+                M.copies.release();
+                return st;
+            }
+        }
+        if (need <= M.copies.n) M.ncopies = want;
+    }
     if (M.layout_poff == poff && M.layout_cnt == cnt && M.ns.p) return KHRR_OK;
     const size_t np = static_cast<size_t>(npad);
-    khrr_status st;
     if ((st = cuda(M.pci.ensure(np), "alloc")) != KHRR_OK) return st;
     if ((st = cuda(M.part.ensure(np), "alloc")) != KHRR_OK) return st;
     if ((st = cuda(M.ns.ensure(np), "alloc")) != KHRR_OK) return st;
@@ -636,7 +675,7 @@ khrr_status khrr_ctx::mesh_enqueue_force(const double* x, int iters, int rot0) {
     if ((st = cuda(cudaMemsetAsync(M.cell_mass.p, 0, cz * sizeof(double), s), "memset")) != KHRR_OK) return st;
     for (size_t k = 0; k < cnt.size(); ++k) {
         const int64_t o = poff[k];
-        cudaError_t e = cic ? launch_cic_deposit(x + 3 * o, mass.p + o, cnt[k], M.geom, M.cell_mass.p, s)
+        cudaError_t e = cic ? launch_cic_deposit(x + 3 * o, mass.p + o, cnt[k], M.geom, M.cell_mass.p, M.copies.p, M.ncopies, s)
                             : launch_assign_cells(x + 3 * o, cnt[k], M.geom, M.pci.p + o, mass.p + o, M.cell_mass.p, s);
         if ((st = cuda(e, "deposit")) != KHRR_OK) return st;
     }
