@@ -337,6 +337,37 @@ void plan_pair_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, 
                      [](const PairItem& a, const PairItem& b) { return a.cost > b.cost; });
 }
 
+// One item per 128 x ki bodies and later block (or their own), and one per
+// later tile of every block; the longer i-side items first.
+void plan_small_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int sms, ForcePlan& out) {
+    out.small_items.clear();
+    out.small_ki = 0;
+    const int64_t pairs = static_cast<int64_t>(out.pair_items.size());
+    // Up to 78 block pairs (12 blocks, 12,288 bodies) on 148 SMs; two bodies
+    // per thread from eight blocks on (one / two: 33 / 47 us at 6,144 bodies,
+    // 51 / 52 at 8,192, 76 / 68 at 10,007).
+    if (5 * pairs > 3 * sms) return;
+    out.small_ki = 5 * pairs > sms ? 2 : 1;
+    for (size_t k = 0; k < cnt.size(); ++k) {
+        const std::vector<int64_t>& bb = blocks[k];
+        const int real_end = static_cast<int>(bb[0] + cnt[k]);
+        for (size_t b = 0; b + 1 < bb.size(); ++b)
+            for (size_t J = b; J + 1 < bb.size(); ++J)
+                for (int64_t i = bb[b]; i < bb[b + 1]; i += kPairThreads * out.small_ki)
+                    out.small_items.push_back(SmallItem{
+                        0, static_cast<int>(i), static_cast<int>(std::min(i + kPairThreads * out.small_ki, bb[b + 1])),
+                        static_cast<int>(bb[J]), static_cast<int>(bb[J + 1]), real_end});
+    }
+    for (size_t k = 0; k < cnt.size(); ++k) {
+        const std::vector<int64_t>& bb = blocks[k];
+        const int real_end = static_cast<int>(bb[0] + cnt[k]);
+        for (size_t b = 0; b + 1 < bb.size(); ++b)
+            for (int64_t j = bb[b + 1]; j < bb.back(); j += kPairTile)
+                out.small_items.push_back(SmallItem{1, static_cast<int>(bb[b]), static_cast<int>(bb[b + 1]),
+                                                    static_cast<int>(j), static_cast<int>(j + kPairTile), real_end});
+    }
+}
+
 // A CTA takes as long for a short i block as for a full one, so the time goes
 // with the j tiles (the i block's own tiles: 11 packed operations against 14).
 void weigh_pair_items(int sms, ForcePlan& out) {
@@ -452,6 +483,8 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
         if (p.valid && p.pair && p.split_req == tuning.j_split && p.ctas == ctas) return KHRR_OK;
         plan_pair_items(pair_blocks, cnt, ctas, tuning.j_split, p);
         weigh_pair_items(sm_count, p);
+        p.small_ki = 0;
+        if (tuning.j_split == 0) plan_small_items(pair_blocks, cnt, sm_count, p);
         p.pair = true;
         p.threads = v->threads;
         p.ipt = v->i_per_thread;
@@ -462,6 +495,12 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
         if ((st = cuda(cudaMemcpyAsync(p.d_pair_items.p, p.pair_items.data(), p.pair_items.size() * sizeof(PairItem),
                                        cudaMemcpyHostToDevice, stream),
                        "upload items")) != KHRR_OK)
+            return st;
+        if (p.small_ki &&
+            ((st = cuda(p.d_small_items.ensure(p.small_items.size()), "alloc items")) != KHRR_OK ||
+             (st = cuda(cudaMemcpyAsync(p.d_small_items.p, p.small_items.data(),
+                                        p.small_items.size() * sizeof(SmallItem), cudaMemcpyHostToDevice, stream),
+                        "upload items")) != KHRR_OK))
             return st;
         if ((st = cuda(fx.ensure(static_cast<size_t>(kFxComps) * npad), "alloc fixed-point sums")) != KHRR_OK)
             return st;
@@ -620,7 +659,10 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
         a.h_uniform = h_uniform;
         a.tile_mass = tile_mass.p;
         a.err = errflag.p;
-        if ((st = cuda(launch_pair(v, a, std::min(a.n_items, ctas), stream), "pair force kernel")) != KHRR_OK)
+        if ((st = cuda(p.small_ki ? launch_pair_small(v, a, p.d_small_items.p, static_cast<int>(p.small_items.size()),
+                                                      p.small_ki, stream)
+                                  : launch_pair(v, a, std::min(a.n_items, ctas), sm_count, stream),
+                       "pair force kernel")) != KHRR_OK)
             return st;
     } else {
         const int e = static_cast<int>(p.items.size());

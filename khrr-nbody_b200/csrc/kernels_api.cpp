@@ -62,6 +62,8 @@ khrr_status prepare_pair_pass(khrr_ctx* c, const double* mass, const double* eps
         std::vector<int64_t> cnt{n};
         plan_pair_items(pair_blocks_fixed({0, npad}), cnt, ctas, c->tuning.j_split, p);
         weigh_pair_items(c->sm_count, p);
+        p.small_ki = 0;
+        if (c->tuning.j_split == 0) plan_small_items(pair_blocks_fixed({0, npad}), cnt, c->sm_count, p);
         p.pair = true;
         p.threads = v->threads;
         p.ipt = v->i_per_thread;
@@ -72,6 +74,11 @@ khrr_status prepare_pair_pass(khrr_ctx* c, const double* mass, const double* eps
         if ((st = c->cuda(cudaMemcpy(p.d_pair_items.p, p.pair_items.data(), p.pair_items.size() * sizeof(PairItem),
                                      cudaMemcpyHostToDevice),
                           "upload items")) != KHRR_OK)
+            return st;
+        if (p.small_ki && ((st = c->cuda(p.d_small_items.ensure(p.small_items.size()), "alloc")) != KHRR_OK ||
+                           (st = c->cuda(cudaMemcpy(p.d_small_items.p, p.small_items.data(),
+                                                    p.small_items.size() * sizeof(SmallItem), cudaMemcpyHostToDevice),
+                                         "upload items")) != KHRR_OK))
             return st;
         p.valid = true;
         c->kplan_n = n;
@@ -172,8 +179,10 @@ khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i)
                           "sums reset")) != KHRR_OK)
             return st;
         if (e0) cudaEventRecord(e0, s);
-        if ((st = c->cuda(launch_pair(v, a, std::min(a.n_items, c->resident_ctas(v)), s), "pair force kernel")) !=
-            KHRR_OK)
+        if ((st = c->cuda(p.small_ki ? launch_pair_small(v, a, p.d_small_items.p, static_cast<int>(p.small_items.size()),
+                                                         p.small_ki, s)
+                                     : launch_pair(v, a, std::min(a.n_items, c->resident_ctas(v)), c->sm_count, s),
+                          "pair force kernel")) != KHRR_OK)
             return st;
         if (e1) cudaEventRecord(e1, s);
         if (c->timing) {

@@ -118,6 +118,7 @@ struct PairArgs {
     int n_items;
     unsigned* queue;         // kQueueWords words (zeroed before each launch)
     unsigned share;          // an SM's share of the items' weight
+    unsigned may_stop;       // CTAs that may stop at it (set by launch_pair)
     unsigned long long* fx;  // fixed-point sums [kFxComps][npad] (zeroed before each launch)
     long long npad;          // component stride
     const FxScale* scale;    // per 128-body tile
@@ -126,10 +127,21 @@ struct PairArgs {
     unsigned* err;           // device error flag word
 };
 
+// One unit of the small-layout form (pair_small.cu), padded device indices.
+// kind 0: the i-side sums of bodies [i_begin, i_end) (at most NT x KI of one
+// block) over the block [j_begin, j_end); kind 1: the reactions of the block
+// [i_begin, i_end) on the tile [j_begin, j_end).
+struct SmallItem {
+    int kind, i_begin, i_end, j_begin, j_end, real_end;
+};
+// v: the pair variant whose sums are wanted (its outputs and form).
+cudaError_t launch_pair_small(const ForceVariant* v, const PairArgs& a, const SmallItem* items, int n, int ki,
+                              cudaStream_t s);
+
 int pair_variant_count();
 const ForceVariant* pair_variant(int idx);
 const ForceVariant* find_pair_variant(bool unif, bool acc, bool phi, bool block_mass);
-cudaError_t launch_pair(const ForceVariant* v, const PairArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_pair(const ForceVariant* v, const PairArgs& a, int grid, int sms, cudaStream_t s);
 // Fixed-point sums -> acc[i] (+)= a_i and/or phi[i] (-)= sum m/r, i < n (FP64).
 cudaError_t launch_reduce_pair_fx(const unsigned long long* fx, long long npad, const FxScale* scale, int64_t n,
                                   double* acc, double* phi, bool overwrite, cudaStream_t s);

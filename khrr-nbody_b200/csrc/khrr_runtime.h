@@ -68,6 +68,10 @@ struct ForcePlan {
     bool f64_pair = false;  // FP64 plan: the symmetric FP64 kernel on pair_items
     std::vector<PairItem> pair_items;
     unsigned pair_share = 0;  // an SM's share of the items' weight
+    // The same work in the small-layout form, where that is the faster one.
+    int small_ki = 0;  // i bodies per thread (0: the pair kernel runs)
+    std::vector<SmallItem> small_items;
+    DevBuf<SmallItem> d_small_items;
     DevBuf<PairItem> d_pair_items;
     ForcePlan() = default;
     ForcePlan(const ForcePlan&) = delete;
@@ -86,6 +90,9 @@ PairBlocks pair_blocks_fixed(const std::vector<int64_t>& poff);
 PairBlocks pair_blocks_by_mass(const std::vector<int64_t>& poff, const std::vector<float>& tile_mass);
 // The pair kernel's items: block rows cut into chunks of `chunk` blocks (0 =
 // chosen from the CTA count), costliest first.
+// The pair plan's work in the small-layout form, or small_ki = 0.  Called on
+// plans whose items are single block pairs.
+void plan_small_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int sms, ForcePlan& out);
 // Time weights of a pair plan's items, heaviest first, and the share of one of
 // `sms` SMs.
 void weigh_pair_items(int sms, ForcePlan& out);

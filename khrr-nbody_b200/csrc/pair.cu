@@ -57,37 +57,10 @@
 
 #include "async_copy.cuh"
 #include "khrr_internal.h"
+#include "pair_math.cuh"
 
 namespace khrr {
 namespace {
-
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-__device__ __forceinline__ void two_sum_into(float& hi, float& lo, float p) {
-    const float s = hi + p;
-    const float bp = s - hi;
-    const float e = (hi - (s - bp)) + (p - bp);
-    hi = s;
-    lo += e;
-}
-
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-
-// A partial (FP32) as a fixed-point integer: times the power of two s,
-// rounded to the nearest integer (exact for |v s| >= 2^24).
-__device__ __forceinline__ long long to_fx(float v, double s) {
-    return __double2ll_rn(static_cast<double>(v) * s);
-}
-
-// Integer atomic add without return (red.global.add.u64): two's complement
-// makes the unsigned add a signed one.
-__device__ __forceinline__ void fx_add(unsigned long long* p, long long v) {
-    atomicAdd(p, static_cast<unsigned long long>(v));
-}
 
 __device__ __forceinline__ float2 shfl2(float2 v, int src) {
     return f2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
@@ -121,10 +94,6 @@ constexpr int kSUnroll = KHRR_PAIR_UNROLL;
 constexpr int kFoldEvery = KHRR_PAIR_FOLD;
 constexpr int kSUnrollPhi = 1;
 
-constexpr unsigned kUnif = 1;   // every body has the same softening: no h array
-constexpr unsigned kAcc = 2;    // accumulate accelerations
-constexpr unsigned kPhi = 4;    // accumulate potentials
-constexpr unsigned kBMass = 8;  // one mass per block: masses factored out
 // Lanes past a short block's end, in the block-mass form, sit this far away:
 // r^-3 underflows to exactly 0, so they add nothing to the accelerations'
 // reactions, and r^-1 (< 6e-19) adds nothing visible to the potentials'.
@@ -245,8 +214,9 @@ constexpr int pair_min_blocks() {
 // most items does, and CTAs that pull freely finish in step: the SMs whose
 // three come first take three more items each and the others none (1,176
 // items at 49,152 bodies: nine on most SMs where eight on each would do).  So
-// an SM stops pulling once it has taken its share of the weight; the last CTA
-// of the grid never stops, whatever the shares and wherever the CTAs run.
+// an SM stops pulling once it has taken its share of the weight.  As many
+// CTAs as there are SMs never stop, whatever the shares and wherever the CTAs
+// run: they finish what the shares, rounded to items, leave over.
 // Per acceleration pass 684 -> 627 us at 49,152 bodies, 327 -> 307 at 30,720,
 // 4302 -> 4213 at 131,072; from 786k on (0.1 %) it makes no difference.
 __device__ __forceinline__ int next_item(const PairArgs& a) {
@@ -255,7 +225,7 @@ __device__ __forceinline__ int next_item(const PairArgs& a) {
     const unsigned ahead = *reinterpret_cast<volatile unsigned*>(a.queue);
     if (ahead >= static_cast<unsigned>(a.n_items)) return a.n_items;
     const unsigned taken = atomicAdd(a.queue + kQueueLoad + sm % kQueueSms, static_cast<unsigned>(a.items[ahead].weight));
-    if (taken >= a.share && atomicAdd(a.queue + kQueueStopped, 1u) + 1u < gridDim.x) return a.n_items;
+    if (taken >= a.share && atomicAdd(a.queue + kQueueStopped, 1u) < a.may_stop) return a.n_items;
     return static_cast<int>(atomicAdd(a.queue, 1u));
 }
 
@@ -645,8 +615,9 @@ cudaError_t launch_classify(const double* mass, const double* eps2, int64_t n, f
     return cudaGetLastError();
 }
 
-cudaError_t launch_pair(const ForceVariant* v, const PairArgs& a, int grid, cudaStream_t s) {
+cudaError_t launch_pair(const ForceVariant* v, const PairArgs& a, int grid, int sms, cudaStream_t s) {
     PairArgs args = a;
+    args.may_stop = grid > sms ? static_cast<unsigned>(grid - sms) : 0u;
     void* params[] = {&args};
     return cudaLaunchKernel(v->fn, dim3(grid), dim3(v->threads), params, v->smem, s);
 }
