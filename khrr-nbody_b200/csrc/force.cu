@@ -162,11 +162,13 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
     };
 
     unsigned consumed = 0;  // tiles this CTA has consumed, over all its items
-    for (;;) {
-        if (tid == 0) s_item = static_cast<int>(atomicAdd(a.queue, 1u));
-        __syncthreads();
-        const int it = s_item;
-        if (it >= a.n_items) break;
+    // The first item is the CTA's own, the queue gives the ones after the
+    // grid's: with no more items than CTAs nothing waits for the queue (two
+    // round trips to L2 in a pass of a few microseconds: with the corrector's
+    // loads ahead 14.3 -> 12.3 us per time step of 3,072 bodies).
+    const int grid = static_cast<int>(gridDim.x);
+    int it = static_cast<int>(blockIdx.x);
+    while (it < a.n_items) {
         const WorkItem w = a.items[it];
         const int ntiles = (w.j_end - w.j_begin) / JT;
         if (tid == 0) {
@@ -332,6 +334,12 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
                 out[i] = o;
             }
         }
+        if (a.n_items <= grid) break;
+        // Every thread has read the last item's number: the tile loop's
+        // barriers lie in between (an item has at least one tile).
+        if (tid == 0) s_item = grid + static_cast<int>(atomicAdd(a.queue, 1u));
+        __syncthreads();
+        it = s_item;
     }
 }
 

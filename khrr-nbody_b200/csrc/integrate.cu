@@ -131,13 +131,23 @@ __device__ __forceinline__ void sum_partials(const StepArgs& a, int64_t i, d3& s
         for (int c = 0; c < 8; ++c) u[c * a.npad] = 0.0;
         return;
     }
+    // Slots in order, eight loads in flight (a small system's 24 slots one
+    // after the other took most of the corrector's 8 us).
     const int ns = a.nsplit[i];
-    for (int k = 0; k < ns; ++k) {
-        const double4 p = a.part[k * a.npad + i];
-        s.x += p.x;
-        s.y += p.y;
-        s.z += p.z;
-        sp += p.w;
+    constexpr int kAhead = 8;
+    for (int k0 = 0; k0 < ns; k0 += kAhead) {
+        double4 p[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (k0 + k < ns) p[k] = a.part[(k0 + k) * a.npad + i];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (k0 + k < ns) {
+                s.x += p[k].x;
+                s.y += p[k].y;
+                s.z += p[k].z;
+                sp += p[k].w;
+            }
     }
 }
 
@@ -302,6 +312,10 @@ __global__ void __launch_bounds__(kConsThreads) conservation_kernel(const double
     }
 }
 
+// Threads per block of the per-body kernels: 256, or 64 where that leaves SMs
+// without a block.
+int step_block(int64_t n) { return n < 148 * 256 ? 64 : 256; }
+
 int grid_for(int64_t n, int block) {
     int64_t g = (n + block - 1) / block;
     if (g > 148 * 16) g = 148 * 16;
@@ -312,17 +326,20 @@ int grid_for(int64_t n, int block) {
 }  // namespace
 
 cudaError_t launch_predictor(const StepArgs& a, cudaStream_t s) {
-    predictor_kernel<<<grid_for(a.n, 256), 256, 0, s>>>(a);
+    const int b = step_block(a.n);
+    predictor_kernel<<<grid_for(a.n, b), b, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_corrector(const StepArgs& a, cudaStream_t s) {
-    corrector_kernel<<<grid_for(a.n, 256), 256, 0, s>>>(a);
+    const int b = step_block(a.n);
+    corrector_kernel<<<grid_for(a.n, b), b, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_collect(const StepArgs& a, bool want_acc, bool accumulate, cudaStream_t s) {
-    collect_kernel<<<grid_for(a.n, 256), 256, 0, s>>>(a, want_acc ? 1 : 0, accumulate ? 1 : 0);
+    const int b = step_block(a.n);
+    collect_kernel<<<grid_for(a.n, b), b, 0, s>>>(a, want_acc ? 1 : 0, accumulate ? 1 : 0);
     return cudaGetLastError();
 }
 
