@@ -119,11 +119,18 @@ khrr_status khrr_ctx::cuda(cudaError_t e, const char* what) {
     return fail(KHRR_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+// Waits for the stream.  The flag's copy goes to page-locked memory behind the
+// stream's work, so one wait covers both (a second wait for a pageable copy
+// took 12 us more).
 khrr_status khrr_ctx::check_device_flag() {
-    unsigned flag = 0;
-    cudaError_t e = cudaMemcpyAsync(&flag, errflag.p, sizeof flag, cudaMemcpyDeviceToHost, stream);
+    unsigned* flag = reinterpret_cast<unsigned*>(host_words + 16);
+    cudaError_t e = cudaMemcpyAsync(flag, errflag.p, sizeof *flag, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return cuda(e, "device error flag");
+    return report_flag(*flag);
+}
+
+khrr_status khrr_ctx::report_flag(unsigned flag) {
     if (flag & kErrTimeout) {
         cudaMemsetAsync(errflag.p, 0, sizeof(unsigned), stream);
         return fail(KHRR_ERR_TIMEOUT, "a kernel gave up a bounded wait (an asynchronous copy or a neighbour plane)");
@@ -864,7 +871,8 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
         cudaEventCreate(&c->ph0) != cudaSuccess || cudaEventCreate(&c->ph1) != cudaSuccess ||
         c->queue.ensure(kQueueWords) != cudaSuccess || c->errflag.ensure(1) != cudaSuccess ||
         c->cons_done.ensure(1) != cudaSuccess ||
-        c->scratch.ensure(64) != cudaSuccess) {
+        c->scratch.ensure(64) != cudaSuccess ||
+        cudaHostAlloc(reinterpret_cast<void**>(&c->host_words), 17 * sizeof(double), cudaHostAllocDefault) != cudaSuccess) {
         khrr_destroy(c);
         return KHRR_ERR_CUDA;
     }
@@ -903,6 +911,7 @@ void khrr_destroy(khrr_ctx* c) {
     if (c->ph0) cudaEventDestroy(c->ph0);
     if (c->ph1) cudaEventDestroy(c->ph1);
     if (c->own) cudaStreamDestroy(c->own);
+    if (c->host_words) cudaFreeHost(c->host_words);
     delete c;  // device buffers free themselves
 }
 
@@ -923,8 +932,6 @@ khrr_status khrr_set_stream(khrr_ctx* c, void* stream) {
 
 khrr_status khrr_synchronize(khrr_ctx* c) {
     if (!c) return KHRR_ERR_INVALID_ARG;
-    khrr_status st = c->cuda(cudaStreamSynchronize(c->stream), "synchronize");
-    if (st != KHRR_OK) return st;
     return c->check_device_flag();
 }
 
@@ -1263,14 +1270,12 @@ khrr_status khrr_conservation(khrr_ctx* c, khrr_lie* out) {
     khrr_status st;
     if ((st = c->cuda(c->cons_blocks.ensure(static_cast<size_t>(nb) * 16), "alloc")) != KHRR_OK) return st;
     if ((st = c->cuda(launch_conservation(c->pos.p, c->vel.p, c->mass.p, c->phi.p, c->npad, c->cons_blocks.p,
-                                          nb, c->cons_done.p, c->scratch.p, c->stream),
-                      "conservation")) != KHRR_OK)
+                                          nb, c->cons_done.p, c->errflag.p, c->host_words, c->stream),
+                      "conservation")) != KHRR_OK ||
+        (st = c->cuda(cudaStreamSynchronize(c->stream), "synchronize")) != KHRR_OK)
         return st;
-    double v[16];
-    if ((st = c->cuda(cudaMemcpyAsync(v, c->scratch.p, sizeof v, cudaMemcpyDeviceToHost, c->stream), "download")) !=
-        KHRR_OK)
-        return st;
-    if ((st = khrr_synchronize(c)) != KHRR_OK) return st;
+    const double* v = c->host_words;
+    if ((st = c->report_flag(static_cast<unsigned>(v[15]))) != KHRR_OK) return st;
     for (int k = 0; k < 3; ++k) {
         out->L[k] = v[k];
         out->Imp[k] = v[3 + k];

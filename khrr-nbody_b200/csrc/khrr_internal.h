@@ -253,12 +253,13 @@ cudaError_t launch_collect(const StepArgs& a, bool want_acc, bool accumulate, cu
 cudaError_t launch_integ_time(const double* acc, double* pos_t, double* vel_t, const double* pos,
                               const double* vel, double dt, int istep, double* acc0, int64_t n,
                               const FieldConsts& f, cudaStream_t s);
-// FP64 conservation sums over bodies; done: a word that is zero before the
-// call and after it (ghosts have zero mass and contribute
-// nothing to the sums; they sit at the origin with zero velocity).
+// FP64 conservation sums over bodies (ghosts have zero mass and contribute
+// nothing to the sums; they sit at the origin with zero velocity); done: a word
+// that is zero before the call and after it; out16: page-locked host memory or
+// device memory, [15] the value of *err.
 cudaError_t launch_conservation(const double* pos, const double* vel, const double* mass,
                                 const double* phi, int64_t n, double* block_out, int nblocks, unsigned* done,
-                                double* out16, cudaStream_t s);
+                                const unsigned* err, double* out16, cudaStream_t s);
 int conservation_blocks(int64_t n);
 
 // ---- mesh.cu ------------------------------------------------------------------

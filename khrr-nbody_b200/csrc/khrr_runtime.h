@@ -162,6 +162,11 @@ struct khrr_ctx {
     std::vector<khrr::FxScale> fx_scales; // host copy (kept alive until the upload's copies complete)
     khrr::DevBuf<double> f64_sums;  // the symmetric FP64 pass's sums, 2 x 4 x npad
     khrr::DevBuf<unsigned> queue, errflag;
+    // Page-locked words that small results come back through: 16 doubles of
+    // khrr_conservation (the last one the error flag's value), then the error
+    // flag of khrr_synchronize.  Read by the host after a synchronisation.
+    double* host_words = nullptr;
+    khrr_status report_flag(unsigned flag);
     khrr::DevBuf<double> cons_blocks, scratch;
     khrr::DevBuf<unsigned> cons_done;  // khrr_conservation's count of finished blocks (zero between calls)
     bool uniform = false;

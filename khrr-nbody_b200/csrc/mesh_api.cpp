@@ -405,12 +405,11 @@ khrr_status khrr_wave_solve(khrr_ctx* c, const khrr_wave_params* p, double tol, 
         StepGraph* g = nullptr;
         if ((st = chunk_graph(k, c->wave_rot, &g)) != KHRR_OK) return st;
         if ((st = c->cuda(cudaGraphLaunch(g->exec, s), "wave graph")) != KHRR_OK) return st;
-        double r2[2];
-        if ((st = c->cuda(cudaMemcpyAsync(r2, c->wave_resid.p, sizeof r2, cudaMemcpyDeviceToHost, s), "download")) !=
-            KHRR_OK)
+        const double* r2 = c->host_words;
+        if ((st = c->cuda(cudaMemcpyAsync(c->host_words, c->wave_resid.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s),
+                          "download")) != KHRR_OK)
             return st;
-        if ((st = c->cuda(cudaStreamSynchronize(s), "wave sync")) != KHRR_OK) return st;
-        if ((st = c->check_device_flag()) != KHRR_OK) return st;
+        if ((st = c->check_device_flag()) != KHRR_OK) return st;  // waits for the stream
         done += k;
         c->wave_rot = ring_after_f32(c->wave_rot, k);
         rel = r2[1] > 0.0 ? std::sqrt(r2[0] / r2[1]) : (r2[0] > 0.0 ? INFINITY : 0.0);
