@@ -181,7 +181,7 @@ struct khrr_ctx {
     khrr::ForcePlan plan_batched, plan_plain, plan_fp64;
     bool predicted = false;
     double pred_dt = 0.0;
-    std::map<std::tuple<uint64_t, int, bool, bool, bool>, khrr::StepGraph> graphs;  // (dt, mode, phi, compat, timed)
+    std::map<std::tuple<uint64_t, int, int, bool, bool, bool>, khrr::StepGraph> graphs;  // (dt, steps, mode, phi, compat, timed)
     // Every force pass starts from a zero queue counter and, where its kernel
     // accumulates, zero sums; the kernel that reads the sums zeroes both again.
     // clean: the kind of pass they are zero for (0: unknown).
@@ -254,7 +254,7 @@ struct khrr_ctx {
     khrr::StepArgs step_args(const khrr::ForcePlan& p, double dt);
     khrr::Shadow shadow() { return khrr::shadow_at(shadow_buf.p, npad); }
     khrr_status enqueue_step(double dt, int mode, bool phi_now, bool compat, bool events);
-    khrr_status get_step_graph(double dt, int mode, bool phi_now, bool compat, khrr::StepGraph** out);
+    khrr_status get_step_graph(double dt, int nsteps, int mode, bool phi_last, bool compat, khrr::StepGraph** out);
     khrr_status timing_pair(cudaEvent_t* e0, cudaEvent_t* e1);
     khrr_status call_start();  // with timing on: event before the call's first kernel
     khrr_status call_stop();   // with timing on: event after its last kernel
