@@ -25,7 +25,8 @@
 // thread), by shared-memory loads (6-10 per step for one or two bodies) and
 // the FP32 pipe at the large one.  us per acceleration pass, pair kernel ->
 // this (events around the call): 117 -> 28 at 3,072 bodies, 117 -> 33 at 6,144,
-// 139 -> 68 at 10,007 (masses and softenings per body), 119 -> 88 at 12,288;
+// 139 -> 64 at 10,007 (68 without the forms of one mass and softening per
+// tile), 119 -> 88 at 12,288;
 // 120 -> 115 at 14,336, 185 -> 188 at 20,480 (pair kernel kept).
 #include <cstdint>
 
@@ -67,12 +68,84 @@ __device__ __forceinline__ void pair_term(float2 X2, float2 Y2, float2 Z2, float
     i3 = __fmul2_rn(inv, __fmul2_rn(inv, inv));
 }
 
+// One tile of the i side (kind 0).  ONE: the tile's masses are all mt and its
+// softenings with the warp's bodies' add up to e2; the same numbers as the
+// general form without reading and adding them per pair.
+template <unsigned F, int KI, bool ONE>
+__device__ __forceinline__ void side_tile(const float (&sb)[SmallShape<F>::NCOMP][kPairBlock], int t0, int lane,
+                                          const float2 (&nx)[KI], const float2 (&ny)[KI], const float2 (&nz)[KI],
+                                          const float2 (&hi)[KI], float2 e2, float2 mt,
+                                          float2 (&ai)[SmallShape<F>::NC][KI]) {
+    using S = SmallShape<F>;
+    constexpr bool UNIF = S::UNIF || ONE, ACC = S::ACC, PHI = S::PHI, BMASS = S::BMASS;
+    constexpr int CP = S::NC - 1;
+    constexpr int kU = 4 / KI;  // steps in flight: the chains leave only the last FMA serial
+#pragma unroll 1
+    for (int c0 = 0; c0 < JT; c0 += 64) {
+#pragma unroll kU
+        for (int s = 0; s < 32; ++s) {
+            const int ja = t0 + c0 + ((lane + s) & 31), jb = ja + 32;
+            const float2 X2 = f2(sb[0][ja], sb[0][jb]), Y2 = f2(sb[1][ja], sb[1][jb]);
+            const float2 Z2 = f2(sb[2][ja], sb[2][jb]);
+            const float2 M2 = BMASS ? f2(1.f, 1.f) : ONE ? mt : f2(sb[S::kOffM][ja], sb[S::kOffM][jb]);
+            const float2 H2 = UNIF ? f2(0.f, 0.f) : f2(sb[S::kOffH][ja], sb[S::kOffH][jb]);
+#pragma unroll
+            for (int k = 0; k < KI; ++k) {
+                float2 dx, dy, dz, inv, i3;
+                pair_term<UNIF>(X2, Y2, Z2, H2, nx[k], ny[k], nz[k], hi[k], e2, dx, dy, dz, inv, i3);
+                if (ACC) {
+                    const float2 fi = BMASS ? i3 : __fmul2_rn(M2, i3);
+                    ai[0][k] = __ffma2_rn(dx, fi, ai[0][k]);
+                    ai[1][k] = __ffma2_rn(dy, fi, ai[1][k]);
+                    ai[2][k] = __ffma2_rn(dz, fi, ai[2][k]);
+                }
+                if (PHI) ai[CP][k] = BMASS ? __fadd2_rn(ai[CP][k], inv) : __ffma2_rn(M2, inv, ai[CP][k]);
+            }
+        }
+    }
+}
+
+// The chains of the j side (kind 1): the block's n bodies (the warp's 32 of
+// every 128) on the lane's four.  ONE as above, mt the block's mass.
+template <unsigned F, bool ONE>
+__device__ __forceinline__ void reaction_chains(const float (&sb)[SmallShape<F>::NCOMP][kPairBlock], int n, int lane,
+                                                int warp, const float2 (&X2)[2], const float2 (&Y2)[2],
+                                                const float2 (&Z2)[2], const float2 (&H2)[2], float2 e2, float2 mt,
+                                                float2 (&r)[SmallShape<F>::NC][2]) {
+    using S = SmallShape<F>;
+    constexpr bool UNIF = S::UNIF || ONE, ACC = S::ACC, PHI = S::PHI, BMASS = S::BMASS;
+    constexpr int CP = S::NC - 1;
+#pragma unroll 1
+    for (int s = 0; s < 32; ++s) {
+        const int li = warp * 32 + ((lane - s) & 31);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int q = k * NT + li;
+            if (k * NT >= n) break;  // blocks are whole tiles
+            const float2 nx = f2(sb[0][q], sb[0][q]), ny = f2(sb[1][q], sb[1][q]), nz = f2(sb[2][q], sb[2][q]);
+            const float2 mi = BMASS ? f2(1.f, 1.f) : ONE ? mt : f2(sb[S::kOffM][q], sb[S::kOffM][q]);
+            const float2 hi = UNIF ? f2(0.f, 0.f) : f2(sb[S::kOffH][q], sb[S::kOffH][q]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                float2 dx, dy, dz, inv, i3;
+                pair_term<UNIF>(X2[p], Y2[p], Z2[p], H2[p], nx, ny, nz, hi, e2, dx, dy, dz, inv, i3);
+                if (ACC) {
+                    const float2 fj = BMASS ? i3 : __fmul2_rn(mi, i3);
+                    r[0][p] = __ffma2_rn(dx, fj, r[0][p]);
+                    r[1][p] = __ffma2_rn(dy, fj, r[1][p]);
+                    r[2][p] = __ffma2_rn(dz, fj, r[2][p]);
+                }
+                if (PHI) r[CP][p] = BMASS ? __fadd2_rn(r[CP][p], inv) : __ffma2_rn(mi, inv, r[CP][p]);
+            }
+        }
+    }
+}
+
 template <unsigned F, int KI>
 __global__ void __launch_bounds__(NT) pair_small_kernel(const PairArgs a, const SmallItem* __restrict__ items) {
     using S = SmallShape<F>;
     constexpr bool UNIF = S::UNIF, ACC = S::ACC, PHI = S::PHI, BMASS = S::BMASS;
     constexpr int NC = S::NC, CP = NC - 1;
-    constexpr int kU = 4 / KI;  // steps in flight: the chains leave only the last FMA serial
     static_assert(NC > 0, "nothing to accumulate");
     __shared__ float sb[S::NCOMP][kPairBlock];
     __shared__ float jw[W][NC][JT];
@@ -114,30 +187,30 @@ __global__ void __launch_bounds__(NT) pair_small_kernel(const PairArgs a, const 
             }
         }
         const float mt = BMASS ? a.tile_mass[w.j_begin / JT] : 1.f;
-        for (int t0 = 0; t0 < n; t0 += JT) {
-#pragma unroll 1
-            for (int c0 = 0; c0 < JT; c0 += 64) {
-#pragma unroll kU
-                for (int s = 0; s < 32; ++s) {
-                    const int ja = t0 + c0 + ((lane + s) & 31), jb = ja + 32;
-                    const float2 X2 = f2(sb[0][ja], sb[0][jb]), Y2 = f2(sb[1][ja], sb[1][jb]);
-                    const float2 Z2 = f2(sb[2][ja], sb[2][jb]);
-                    const float2 M2 = BMASS ? f2(1.f, 1.f) : f2(sb[S::kOffM][ja], sb[S::kOffM][jb]);
-                    const float2 H2 = UNIF ? f2(0.f, 0.f) : f2(sb[S::kOffH][ja], sb[S::kOffH][jb]);
+        const float h0 = __shfl_sync(0xffffffffu, hi[0].x, 0);
+        bool one = true;  // the warp's bodies share a softening (lanes past the end have none)
 #pragma unroll
-                    for (int k = 0; k < KI; ++k) {
-                        float2 dx, dy, dz, inv, i3;
-                        pair_term<UNIF>(X2, Y2, Z2, H2, nx[k], ny[k], nz[k], hi[k], e2, dx, dy, dz, inv, i3);
-                        if (ACC) {
-                            const float2 fi = BMASS ? i3 : __fmul2_rn(M2, i3);
-                            ai[0][k] = __ffma2_rn(dx, fi, ai[0][k]);
-                            ai[1][k] = __ffma2_rn(dy, fi, ai[1][k]);
-                            ai[2][k] = __ffma2_rn(dz, fi, ai[2][k]);
-                        }
-                        if (PHI) ai[CP][k] = BMASS ? __fadd2_rn(ai[CP][k], inv) : __ffma2_rn(M2, inv, ai[CP][k]);
-                    }
+        for (int k = 0; k < KI; ++k) one = one && w.i_begin + k * NT + tid < w.i_end && hi[k].x == h0;
+        one = __all_sync(0xffffffffu, one);
+        for (int t0 = 0; t0 < n; t0 += JT) {
+            // One mass and one softening in the tile?
+            float ht = 0.f, m1 = 1.f;
+            bool t_one = one && !(UNIF && BMASS);
+            if (t_one) {
+                if (!UNIF) ht = sb[S::kOffH][t0];
+                if (!BMASS) m1 = sb[S::kOffM][t0];
+#pragma unroll
+                for (int q = 0; q < JT; q += 32) {
+                    if (!UNIF) t_one = t_one && sb[S::kOffH][t0 + q + lane] == ht;
+                    if (!BMASS) t_one = t_one && sb[S::kOffM][t0 + q + lane] == m1;
                 }
+                t_one = __all_sync(0xffffffffu, t_one);
             }
+            if (t_one)
+                side_tile<F, KI, true>(sb, t0, lane, nx, ny, nz, hi, UNIF ? e2 : __fadd2_rn(f2(ht, ht), hi[0]),
+                                       f2(m1, m1), ai);
+            else
+                side_tile<F, KI, false>(sb, t0, lane, nx, ny, nz, hi, e2, f2(1.f, 1.f), ai);
             if (PHI) {  // the potential variants fold every tile
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
@@ -184,30 +257,26 @@ __global__ void __launch_bounds__(NT) pair_small_kernel(const PairArgs a, const 
 #pragma unroll
         for (int c = 0; c < NC; ++c) r[c][p] = f2(0.f, 0.f);
     }
-#pragma unroll 1
-    for (int s = 0; s < 32; ++s) {
-        const int li = warp * 32 + ((lane - s) & 31);
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int q = k * NT + li;
-            if (k * NT >= n) break;  // blocks are whole tiles
-            const float2 nx = f2(sb[0][q], sb[0][q]), ny = f2(sb[1][q], sb[1][q]), nz = f2(sb[2][q], sb[2][q]);
-            const float2 mi = BMASS ? f2(1.f, 1.f) : f2(sb[S::kOffM][q], sb[S::kOffM][q]);
-            const float2 hi = UNIF ? f2(0.f, 0.f) : f2(sb[S::kOffH][q], sb[S::kOffH][q]);
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                float2 dx, dy, dz, inv, i3;
-                pair_term<UNIF>(X2[p], Y2[p], Z2[p], H2[p], nx, ny, nz, hi, e2, dx, dy, dz, inv, i3);
-                if (ACC) {
-                    const float2 fj = BMASS ? i3 : __fmul2_rn(mi, i3);
-                    r[0][p] = __ffma2_rn(dx, fj, r[0][p]);
-                    r[1][p] = __ffma2_rn(dy, fj, r[1][p]);
-                    r[2][p] = __ffma2_rn(dz, fj, r[2][p]);
-                }
-                if (PHI) r[CP][p] = BMASS ? __fadd2_rn(r[CP][p], inv) : __ffma2_rn(mi, inv, r[CP][p]);
-            }
+    // One softening among the tile's bodies and the warp's of the block, and one
+    // mass among the latter?  (A block is whole tiles.)
+    float hb = 0.f, m1 = 1.f;
+    bool one = !(UNIF && BMASS);
+    if (one) {
+        const float hj = __shfl_sync(0xffffffffu, H2[0].x, 0);
+        if (!UNIF) hb = sb[S::kOffH][warp * 32];
+        if (!BMASS) m1 = sb[S::kOffM][warp * 32];
+        if (!UNIF) one = H2[0].x == hj && H2[0].y == hj && H2[1].x == hj && H2[1].y == hj;
+        for (int q = warp * 32 + lane; q < n; q += NT) {
+            if (!UNIF) one = one && sb[S::kOffH][q] == hb;
+            if (!BMASS) one = one && sb[S::kOffM][q] == m1;
         }
+        one = __all_sync(0xffffffffu, one);
     }
+    if (one)
+        reaction_chains<F, true>(sb, n, lane, warp, X2, Y2, Z2, H2, UNIF ? e2 : __fadd2_rn(H2[0], f2(hb, hb)), f2(m1, m1),
+                                 r);
+    else
+        reaction_chains<F, false>(sb, n, lane, warp, X2, Y2, Z2, H2, e2, f2(1.f, 1.f), r);
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
