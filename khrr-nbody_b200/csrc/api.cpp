@@ -349,12 +349,39 @@ void plan_pair_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, 
 void plan_small_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int sms, ForcePlan& out) {
     out.small_items.clear();
     out.small_ki = 0;
-    const int64_t pairs = static_cast<int64_t>(out.pair_items.size());
-    // Up to 78 block pairs (12 blocks, 12,288 bodies) on 148 SMs; two bodies
-    // per thread from eight blocks on (one / two: 33 / 47 us at 6,144 bodies,
-    // 51 / 52 at 8,192, 76 / 68 at 10,007).
-    if (5 * pairs > 3 * sms) return;
-    out.small_ki = 5 * pairs > sms ? 2 : 1;
+    int64_t pairs = 0;
+    for (size_t k = 0; k < cnt.size(); ++k) {
+        const int64_t nb = static_cast<int64_t>(blocks[k].size()) - 1;
+        pairs += nb * (nb + 1) / 2;
+    }
+    if (pairs != static_cast<int64_t>(out.pair_items.size())) return;  // chunks of several blocks
+    // The pair kernel takes a fixed time while every SM has one block pair, and
+    // another while it has two; this form's time goes with their number, less
+    // one where the pair kernel's own term is longer.  us per acceleration
+    // pass, pair kernel / this: of one mass per block 115 / 96 at 13,312
+    // bodies, 115 / 119 at 15,360, 179 / 156 at 17,408, 179 / 189 at 20,480;
+    // otherwise 148 / 97 at 12,500, 148 / 137 at 15,900, 219 / 189 at 20,000,
+    // 219 / 219 at 22,000.
+    const double per_sm = static_cast<double>(pairs) / sms;
+    if (!(per_sm <= 0.95 || (per_sm > 1.0 && per_sm <= 1.6))) return;
+    out.small_one_mass = per_sm <= 0.78 || (per_sm > 1.0 && per_sm <= 1.3);
+    // Two bodies per thread read the tile half as often, one splits the work
+    // finer: two only where they bring the items down to four per SM, or with
+    // more than eight (us per acceleration pass for one / two: 49 / 56 at 7,777
+    // bodies, 51 / 54 at 8,192, 60 / 56 at 8,705, 70 / 63 at 9,500 to 10,007,
+    // 78 / 80 at 10,500, 85 / 88 at 12,288, 101 / 96 at 13,312, 154 / 146 at
+    // 16,999).
+    int64_t items = 0, iside = 0;
+    for (size_t k = 0; k < cnt.size(); ++k) {
+        const std::vector<int64_t>& bb = blocks[k];
+        const int64_t nb = static_cast<int64_t>(bb.size()) - 1;
+        for (int64_t b = 0; b < nb; ++b) {
+            iside += (nb - b) * ((bb[b + 1] - bb[b]) / kPairThreads);
+            items += (bb.back() - bb[b + 1]) / kPairTile;
+        }
+    }
+    const bool four = items + iside > 4 * sms && items + iside / 2 <= 4 * sms;
+    out.small_ki = four || items + iside > 8 * sms ? 2 : 1;
     for (size_t k = 0; k < cnt.size(); ++k) {
         const std::vector<int64_t>& bb = blocks[k];
         const int real_end = static_cast<int>(bb[0] + cnt[k]);
@@ -666,7 +693,7 @@ khrr_status khrr_ctx::enqueue_force(int mode, bool acc, bool phi, bool events, c
         a.h_uniform = h_uniform;
         a.tile_mass = tile_mass.p;
         a.err = errflag.p;
-        if ((st = cuda(p.small_ki ? launch_pair_small(v, a, p.d_small_items.p, static_cast<int>(p.small_items.size()),
+        if ((st = cuda(p.use_small(v) ? launch_pair_small(v, a, p.d_small_items.p, static_cast<int>(p.small_items.size()),
                                                       p.small_ki, stream)
                                   : launch_pair(v, a, std::min(a.n_items, ctas), sm_count, stream),
                        "pair force kernel")) != KHRR_OK)

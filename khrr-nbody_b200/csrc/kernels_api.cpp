@@ -179,7 +179,7 @@ khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i)
                           "sums reset")) != KHRR_OK)
             return st;
         if (e0) cudaEventRecord(e0, s);
-        if ((st = c->cuda(p.small_ki ? launch_pair_small(v, a, p.d_small_items.p, static_cast<int>(p.small_items.size()),
+        if ((st = c->cuda(p.use_small(v) ? launch_pair_small(v, a, p.d_small_items.p, static_cast<int>(p.small_items.size()),
                                                          p.small_ki, s)
                                      : launch_pair(v, a, std::min(a.n_items, c->resident_ctas(v)), c->sm_count, s),
                           "pair force kernel")) != KHRR_OK)

@@ -70,6 +70,8 @@ struct ForcePlan {
     unsigned pair_share = 0;  // an SM's share of the items' weight
     // The same work in the small-layout form, where that is the faster one.
     int small_ki = 0;  // i bodies per thread (0: the pair kernel runs)
+    bool small_one_mass = false;  // ... in the block-mass form too
+    bool use_small(const ForceVariant* v) const { return small_ki && (small_one_mass || !v->tile_mass); }
     std::vector<SmallItem> small_items;
     DevBuf<SmallItem> d_small_items;
     DevBuf<PairItem> d_pair_items;
@@ -90,8 +92,8 @@ PairBlocks pair_blocks_fixed(const std::vector<int64_t>& poff);
 PairBlocks pair_blocks_by_mass(const std::vector<int64_t>& poff, const std::vector<float>& tile_mass);
 // The pair kernel's items: block rows cut into chunks of `chunk` blocks (0 =
 // chosen from the CTA count), costliest first.
-// The pair plan's work in the small-layout form, or small_ki = 0.  Called on
-// plans whose items are single block pairs.
+// The pair plan's work in the small-layout form, or small_ki = 0 (the pair
+// kernel is faster, or its items are not single block pairs).
 void plan_small_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int sms, ForcePlan& out);
 // Time weights of a pair plan's items, heaviest first, and the share of one of
 // `sms` SMs.

@@ -24,10 +24,10 @@
 // CTA's chains at the small end (512 packed steps, 20 us, with one body per
 // thread), by shared-memory loads (6-10 per step for one or two bodies) and
 // the FP32 pipe at the large one.  us per acceleration pass, pair kernel ->
-// this (events around the call): 117 -> 28 at 3,072 bodies, 117 -> 33 at 6,144,
-// 139 -> 64 at 10,007 (68 without the forms of one mass and softening per
-// tile), 119 -> 88 at 12,288;
-// 120 -> 115 at 14,336, 185 -> 188 at 20,480 (pair kernel kept).
+// this (events around the call): 117 -> 25 at 3,072 bodies, 117 -> 33 at 6,144,
+// 139 -> 63 at 10,007 (masses and softenings per body; 68 without the forms of
+// one mass and softening per tile), 148 -> 97 at 12,500, 115 -> 96 at 13,312,
+// 219 -> 189 at 20,000; the planner has the lines.
 #include <cstdint>
 
 #include "khrr_internal.h"
