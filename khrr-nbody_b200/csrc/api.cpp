@@ -1223,6 +1223,12 @@ khrr_status khrr_forces(khrr_ctx* c, int flags) {
     const bool plain = mode == kModePlain;
     cudaStream_t s = c->stream;
     khrr_status st;
+    // In a capture of the caller's both resets are part of the graph, whatever
+    // ran before its replays, and nothing is known about the memory afterwards.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if ((st = c->cuda(cudaStreamIsCapturing(s, &capture), "capture status")) != KHRR_OK) return st;
+    const bool live = capture == cudaStreamCaptureStatusNone;
+    if (!live) c->clean = 0;
     if ((st = c->ensure_plan(mode)) != KHRR_OK || (st = c->ensure_clean(mode)) != KHRR_OK) return st;
     c->clean = 0;  // until the collect below is on its way
     // Shadow of the current positions (a previous step leaves the predicted ones).
@@ -1243,7 +1249,7 @@ khrr_status khrr_forces(khrr_ctx* c, int flags) {
     sa.want_phi = want_phi ? 1 : 0;
     if ((st = c->cuda(launch_collect(sa, want_acc, (flags & KHRR_COMPAT_ACCUMULATE) != 0, s), "collect")) != KHRR_OK)
         return st;
-    c->clean = plain ? 0 : (p.pair ? khrr_ctx::kCleanFx : (p.f64_pair ? khrr_ctx::kCleanF64 : khrr_ctx::kCleanQueue));
+    c->clean = plain || !live ? 0 : (p.pair ? khrr_ctx::kCleanFx : (p.f64_pair ? khrr_ctx::kCleanF64 : khrr_ctx::kCleanQueue));
     c->predicted = false;
     return KHRR_OK;
 }
