@@ -126,6 +126,7 @@ struct MeshSolver {
     DevBuf<double> cell_mass, phi64, cell_acc;  // C, 4 C (field ring), 3 C
     DevBuf<double> copies;                      // cic_copy_count meshes: zero between deposits
     int ncopies = 0;
+    size_t copies_refused = ~size_t(0);         // words that the device had no room for (asked once)
     DevBuf<float> mass32, phi32, tab;           // C, 4 C (field ring), 3 nx
     DevBuf<int2> pci;                           // npad
     DevBuf<double4> part;                       // npad: {acc, -phi} per body
@@ -213,6 +214,7 @@ struct khrr_ctx {
     khrr::DevBuf<double> cell_mass, cell_phi, wave_resid;
     khrr::DevBuf<double> cic_copies;                     // khrr_cic_deposit's extra meshes, zero between calls
     bool cic_deposited = false;                          // a deposit was made without them
+    size_t cic_refused = ~size_t(0);                     // words that the device had no room for (asked once)
     int64_t cell_phi_cells = 0;                          // mesh size the cell_phi sums belong to
     khrr::DevBuf<float> wave_phi, wave_mass, wave_tab;   // 4 C (field ring), C, 3 nx
     int wave_nx = 0;

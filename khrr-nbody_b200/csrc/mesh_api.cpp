@@ -496,14 +496,16 @@ khrr_status khrr_cic_deposit(khrr_ctx* c, const double* pos, const double* mass,
     if (capture != cudaStreamCaptureStatusNone) copies = 0;
     if (copies > 0) {
         const size_t need = static_cast<size_t>(copies) * static_cast<size_t>(C);
-        if (c->cic_copies.n < need && !c->cic_deposited) {
+        if (c->cic_copies.n < need && (!c->cic_deposited || need >= c->cic_refused)) {
             // Allocating them takes as long as some twenty deposits save: from
-            // the context's second deposit on.
+            // the context's second deposit on, and not again where the device
+            // had no room.
             c->cic_deposited = true;
             copies = 0;
         } else if (c->cic_copies.n < need) {
             if (c->cic_copies.ensure(need) != cudaSuccess) {
                 (void)cudaGetLastError();  // no room: deposit directly
+                c->cic_refused = need;
                 copies = 0;
             } else if ((st = c->cuda(cudaMemsetAsync(c->cic_copies.p, 0, need * sizeof(double), c->stream), "memset")) !=
                        KHRR_OK) {
@@ -629,7 +631,8 @@ khrr_status khrr_ctx::mesh_ensure_layout() {
     // attract each other through it.
     if (cnt.size() != 1) return fail(KHRR_ERR_INVALID_ARG, "the mesh solver runs one system (got %zu)", cnt.size());
     khrr_status st;
-    const int want = M.cfg.assign == KHRR_ASSIGN_CIC ? cic_copy_count(cnt[0], M.cells) : 0;
+    int want = M.cfg.assign == KHRR_ASSIGN_CIC ? cic_copy_count(cnt[0], M.cells) : 0;
+    if (static_cast<size_t>(want) * static_cast<size_t>(M.cells) >= M.copies_refused) want = 0;
     const size_t need = static_cast<size_t>(want) * static_cast<size_t>(M.cells);
     if (want != M.ncopies || need > M.copies.n) {
         M.drop_graphs();
@@ -637,6 +640,7 @@ khrr_status khrr_ctx::mesh_ensure_layout() {
         if (need > M.copies.n) {
             if (M.copies.ensure(need) != cudaSuccess) {
                 (void)cudaGetLastError();  // no room: deposit directly
+                M.copies_refused = need;
             } else if ((st = cuda(cudaMemsetAsync(M.copies.p, 0, need * sizeof(double), stream), "memset")) != KHRR_OK) {
                 M.copies.release();
                 return st;
