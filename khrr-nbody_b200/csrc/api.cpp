@@ -187,6 +187,7 @@ void plan_force_items(const std::vector<int64_t>& poff, const std::vector<int64_
     out.sys_item_begin.assign(cnt.size() + 1, 0);
     out.sys_split.assign(cnt.size(), 1);
     out.nslots = 1;
+    out.chains = out.ntiles = 0;
     const size_t nsys = cnt.size();
     std::vector<int> split(nsys, 1);
     double total_cost = 0.0;
@@ -204,28 +205,6 @@ void plan_force_items(const std::vector<int64_t>& poff, const std::vector<int64_
             s = 1;
         } else if (forced_split > 0) {
             s = std::min(forced_split, tiles);
-        } else if (nsys == 1 && 2 * nit * std::max(1, tiles / 8) < ctas) {
-            // Too few bodies for chunks of eight tiles to fill half the grid:
-            // the split with the least estimated time.  An SM's share is its
-            // items times the tiles of one (a CTA alone on an SM reaches 80 %
-            // of the SM's rate), and every chunk's partial sums are written and
-            // read back.  Measured on the packed 128 x 4 shape: 3.7 us per
-            // 128-body tile and SM, ~1 us per item, 64 bytes per slot and body
-            // at 5 TB/s.  Per pass (events around the call, us): 1,000 bodies
-            // 53 -> 15, 3,072 45 -> 15 (144 items instead of 18), 6,144 47 ->
-            // 27, 10,007 95 -> 67; from 14,336 bodies on the rule below is better
-            // (101 against 102; 30,000: 414 against 443).
-            const double tile_us = 3.7 * itile / 512.0;
-            double best = 1e300;
-            for (int c = 1; c <= std::min(64, tiles); ++c) {
-                const double per_sm = std::ceil(static_cast<double>(nit) * c / std::max(sms, 1));
-                const double item = tile_us * std::ceil(static_cast<double>(tiles) / c) + 1.0;
-                const double t = item * (per_sm > 1.0 ? per_sm : 1.25) + 1.3e-5 * c * static_cast<double>(np);
-                if (t < 0.995 * best) {
-                    best = t;
-                    s = c;
-                }
-            }
         } else if (nsys == 1) {
             // Best last-wave fill; chunks of at least 8 tiles; ties -> fewer chunks.
             double best = -1.0;
@@ -239,6 +218,31 @@ void plan_force_items(const std::vector<int64_t>& poff, const std::vector<int64_
                     s = c;
                 }
                 if (eff > 0.985) break;
+            }
+            if (2 * nit * std::max(1, tiles / 8) < ctas) {
+                // Too few bodies for chunks of eight tiles to fill half the
+                // grid: the items are cut finer, by the least estimated time,
+                // and leave one partial per tile, from which the reader forms
+                // the same sums of the s chunks above, bit for bit (a state
+                // whose sums differ in the last bits has bodies rounded to
+                // another FP32 position in its next step, 1e-7 of a velocity
+                // away after a few).  An SM's share is its items times the
+                // tiles of one (a CTA alone on an SM reaches 80 % of the SM's
+                // rate).  Measured on the packed 128 x 4 shape: 3.7 us per
+                // 128-body tile and SM, ~1 us per item.
+                const double tile_us = 3.7 * itile / 512.0;
+                out.chains = s;
+                out.ntiles = tiles;
+                double least = 1e300;
+                for (int c = 1; c <= std::min(64, tiles); ++c) {
+                    const double per_sm = std::ceil(static_cast<double>(nit) * c / std::max(sms, 1));
+                    const double item = tile_us * std::ceil(static_cast<double>(tiles) / c) + 1.0;
+                    const double t = item * (per_sm > 1.0 ? per_sm : 1.25) + 1.3e-5 * c * static_cast<double>(np);
+                    if (t < 0.995 * least) {
+                        least = t;
+                        s = c;
+                    }
+                }
             }
         } else {
             const double target = total_cost / (static_cast<double>(ctas) * 6.0);
@@ -477,6 +481,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
                 return st;
         } else {
             plan_force_items(poff, cnt, kF64ITile, kPad, ctas, sm_count, 0, false, p);
+            p.chains = 0;  // FP64 slots of every chunk
             if ((st = cuda(p.d_items.ensure(p.items.size()), "alloc items")) != KHRR_OK) return st;
             if ((st = cuda(cudaMemcpyAsync(p.d_items.p, p.items.data(), p.items.size() * sizeof(WorkItem),
                                            cudaMemcpyHostToDevice, stream),
@@ -568,7 +573,7 @@ khrr_status khrr_ctx::ensure_plan(int mode) {
     if ((st = cuda(cudaMemcpyAsync(p.d_nsplit.p, ns.data(), ns.size(), cudaMemcpyHostToDevice, stream),
                    "upload nsplit")) != KHRR_OK)
         return st;
-    if ((st = cuda(part.ensure(static_cast<size_t>(p.nslots) * npad), "alloc partials")) != KHRR_OK)
+    if ((st = cuda(part.ensure(p.partial_words(npad)), "alloc partials")) != KHRR_OK)
         return st;
     if ((st = cuda(cudaStreamSynchronize(stream), "plan sync")) != KHRR_OK) return st;
     p.valid = true;
@@ -602,6 +607,7 @@ ForceArgs khrr_ctx::force_args(const ForcePlan& p, int item_begin, int item_end)
     a.n_items = item_end - item_begin;
     a.queue = queue.p;
     a.part = part.p;
+    a.tiles = p.chains > 0 ? reinterpret_cast<float4*>(part.p) : nullptr;
     a.npad = npad;
     a.h_uniform = h_uniform;
     a.tile_mass = tile_mass.p;
@@ -722,6 +728,13 @@ StepArgs khrr_ctx::step_args(const ForcePlan& p, double dt) {
     a.part = part.p;
     a.npad = npad;
     a.nsplit = p.d_nsplit.p;
+    if (!p.pair && p.chains > 0) {
+        const ForceVariant* v = variant(uniform, true, false);
+        a.tiles = reinterpret_cast<const float4*>(part.p);
+        a.ntiles = p.ntiles;
+        a.chains = p.chains;
+        a.tile_mass = v && v->tile_mass ? tile_mass.p : nullptr;
+    }
     a.fx = p.pair ? fx.p : nullptr;
     a.f64 = p.f64_pair ? f64_sums.p : nullptr;
     a.queue = queue.p;

@@ -32,23 +32,10 @@
 
 #include "async_copy.cuh"
 #include "khrr_internal.h"
+#include "tile_sums.cuh"
 
 namespace khrr {
 namespace {
-
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-__device__ __forceinline__ void two_sum_into(float& hi, float& lo, float p) {
-    const float s = hi + p;
-    const float bp = s - hi;
-    const float e = (hi - (s - bp)) + (p - bp);
-    hi = s;
-    lo += e;
-}
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
@@ -162,13 +149,20 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
     };
 
     unsigned consumed = 0;  // tiles this CTA has consumed, over all its items
-    // The first item is the CTA's own, the queue gives the ones after the
-    // grid's: with no more items than CTAs nothing waits for the queue (two
-    // round trips to L2 in a pass of a few microseconds: with the corrector's
-    // loads ahead 14.3 -> 12.3 us per time step of 3,072 bodies).
-    const int grid = static_cast<int>(gridDim.x);
-    int it = static_cast<int>(blockIdx.x);
-    while (it < a.n_items) {
+    // With no more items than CTAs every CTA takes its own and nothing waits for
+    // the queue (two round trips to L2 in a pass of a few microseconds: with
+    // the corrector's loads ahead 14.3 -> 12.3 us per time step of 3,072
+    // bodies).  A first item without the queue for any number of items changed
+    // the compiled loop as well: 1483 -> 1613 us per step of 61,440 bodies with
+    // two softenings.
+    for (;;) {
+        if (tid == 0) {
+            if (a.n_items > static_cast<int>(gridDim.x)) s_item = static_cast<int>(atomicAdd(a.queue, 1u));
+            else s_item = consumed == 0u ? static_cast<int>(blockIdx.x) : a.n_items;
+        }
+        __syncthreads();
+        const int it = s_item;
+        if (it >= a.n_items) break;
         const WorkItem w = a.items[it];
         const int ntiles = (w.j_end - w.j_begin) / JT;
         if (tid == 0) {
@@ -270,31 +264,30 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
                     }
                 }
             }
-            // Fold the tile partials (times the tile mass when it was factored
-            // out) into the compensated running sums.
+            if (a.tiles) {
+                // A few thousand bodies: the runs of tiles that one item sums
+                // below are shared by several, and the reader sums them.
+                float4* out = a.tiles + ((w.j_begin - a.items[0].j_begin) / JT + t) * a.npad;
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                int c = 0;
-                if (ACC) {
-                    float h0 = runr[k][0], l0 = runr[k][1];
-                    two_sum_into(h0, l0, TMASS ? mt * acc.x(k) : acc.x(k));
-                    runr[k][0] = h0;
-                    runr[k][1] = l0;
-                    float h1 = runr[k][2], l1 = runr[k][3];
-                    two_sum_into(h1, l1, TMASS ? mt * acc.y(k) : acc.y(k));
-                    runr[k][2] = h1;
-                    runr[k][3] = l1;
-                    float h2 = runr[k][4], l2 = runr[k][5];
-                    two_sum_into(h2, l2, TMASS ? mt * acc.z(k) : acc.z(k));
-                    runr[k][4] = h2;
-                    runr[k][5] = l2;
-                    c = 3;
+                for (int k = 0; k < K; ++k) {
+                    const int i = w.i_begin + k * NT + tid;
+                    if (i < w.i_end)
+                        out[i] = make_float4(ACC ? acc.x(k) : 0.f, ACC ? acc.y(k) : 0.f, ACC ? acc.z(k) : 0.f,
+                                             PHI ? acc.p(k) : 0.f);
                 }
-                if (PHI) {
-                    float h3 = runr[k][2 * c], l3 = runr[k][2 * c + 1];
-                    two_sum_into(h3, l3, TMASS ? mt * acc.p(k) : acc.p(k));
-                    runr[k][2 * c] = h3;
-                    runr[k][2 * c + 1] = l3;
+            } else {
+                // Fold the tile partials (times the tile mass when it was
+                // factored out) into the compensated running sums.
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const float v[4] = {ACC ? acc.x(k) : 0.f, ACC ? acc.y(k) : 0.f, ACC ? acc.z(k) : 0.f,
+                                        PHI ? acc.p(k) : 0.f};
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const float p = v[ACC ? c : 3];
+                        if (TMASS) two_sum_into(runr[k][2 * c], runr[k][2 * c + 1], mt, p);
+                        else two_sum_into(runr[k][2 * c], runr[k][2 * c + 1], p);
+                    }
                 }
             }
             // Every thread is done with this stage (and all waits ended).
@@ -320,7 +313,7 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int i = w.i_begin + k * NT + tid;
-            if (i < w.i_end) {
+            if (i < w.i_end && !a.tiles) {
                 double4 o;
                 o.x = o.y = o.z = o.w = 0.0;
                 int c = 0;
@@ -334,12 +327,6 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
                 out[i] = o;
             }
         }
-        if (a.n_items <= grid) break;
-        // Every thread has read the last item's number: the tile loop's
-        // barriers lie in between (an item has at least one tile).
-        if (tid == 0) s_item = grid + static_cast<int>(atomicAdd(a.queue, 1u));
-        __syncthreads();
-        it = s_item;
     }
 }
 
@@ -498,6 +485,20 @@ __global__ void reduce_partials_kernel(const double4* __restrict__ part, long lo
     }
 }
 
+__global__ void __launch_bounds__(64) reduce_tiles_kernel(const float4* __restrict__ tiles, long long npad, int ntiles,
+                                                          int chains, int64_t n, double* __restrict__ acc,
+                                                          double* __restrict__ phi, int overwrite) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double4 s = sum_tile_chains<16>(tiles, npad, i, ntiles, chains, nullptr);
+    if (acc) {
+        acc[3 * i] = overwrite ? s.x : acc[3 * i] + s.x;
+        acc[3 * i + 1] = overwrite ? s.y : acc[3 * i + 1] + s.y;
+        acc[3 * i + 2] = overwrite ? s.z : acc[3 * i + 2] + s.z;
+    }
+    if (phi) phi[i] = overwrite ? -s.w : phi[i] - s.w;
+}
+
 // The failure path of the bounded waits, on purpose: one CTA waits on an
 // mbarrier that nothing arrives on (no copy is issued), gives up after
 // limit_ns, raises the error flag and returns like a stalled kernel does.
@@ -623,6 +624,13 @@ cudaError_t launch_reduce_partials(const double4* part, long long npad, int nslo
                                    double* acc, double* phi, bool overwrite, cudaStream_t s) {
     reduce_partials_kernel<<<grid_for(n, 256), 256, 0, s>>>(part, npad, nslots, n, acc, phi,
                                                             overwrite ? 1 : 0);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_reduce_tiles(const float4* tiles, long long npad, int ntiles, int chains, int64_t n, double* acc,
+                                double* phi, bool overwrite, cudaStream_t s) {
+    reduce_tiles_kernel<<<static_cast<unsigned>((n + 63) / 64), 64, 0, s>>>(tiles, npad, ntiles, chains, n, acc, phi,
+                                                                            overwrite ? 1 : 0);
     return cudaGetLastError();
 }
 

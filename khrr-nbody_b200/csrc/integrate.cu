@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "khrr_internal.h"
+#include "tile_sums.cuh"
 
 namespace khrr {
 
@@ -129,6 +130,13 @@ __device__ __forceinline__ void sum_partials(const StepArgs& a, int64_t i, d3& s
         sp = u[3 * a.npad] + l[3 * a.npad];
 #pragma unroll
         for (int c = 0; c < 8; ++c) u[c * a.npad] = 0.0;
+        return;
+    }
+    if (a.tiles) {
+        if (a.nsplit[i] == 0) return;
+        const double4 t = sum_tile_chains<16>(a.tiles, a.npad, i, a.ntiles, a.chains, a.tile_mass);
+        s = d3{t.x, t.y, t.z};
+        sp = t.w;
         return;
     }
     // Slots in order, eight loads in flight (a small system's 24 slots one

@@ -137,7 +137,7 @@ khrr_status prepare_kernel_pass(khrr_ctx* c, const double* pos_i, const double* 
         p.valid = true;
         c->kplan_n = n;
     }
-    if ((st = c->cuda(c->kpart.ensure(static_cast<size_t>(p.nslots) * npad), "alloc partials")) != KHRR_OK)
+    if ((st = c->cuda(c->kpart.ensure(p.partial_words(npad)), "alloc partials")) != KHRR_OK)
         return st;
     cudaStream_t s = c->stream;
     if ((st = c->cuda(launch_pack(pos_j, mass_j, eps2_j, n, npad, shadow_at(c->kshadow.p, npad), s), "pack")) !=
@@ -198,6 +198,7 @@ khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i)
     a.n_items = static_cast<int>(p.items.size());
     a.queue = c->queue.p;
     a.part = c->kpart.p;
+    a.tiles = p.chains > 0 ? reinterpret_cast<float4*>(c->kpart.p) : nullptr;
     a.npad = npad;
     a.h_uniform = 0.0f;
     a.err = c->errflag.p;
@@ -235,6 +236,10 @@ khrr_status khrr_accel(khrr_ctx* c, double* acc, const double* pos_i, const doub
         return c->cuda(launch_reduce_pair_fx(c->kfx.p, round_up(n, kPad), c->kscale.p, n, acc, nullptr,
                                              (flags & KHRR_OVERWRITE) != 0, c->stream),
                        "reduce sums");
+    if (c->kplan.chains > 0)
+        return c->cuda(launch_reduce_tiles(reinterpret_cast<const float4*>(c->kpart.p), round_up(n, kPad), c->kplan.ntiles,
+                                           c->kplan.chains, n, acc, nullptr, (flags & KHRR_OVERWRITE) != 0, c->stream),
+                       "reduce partials");
     return c->cuda(launch_reduce_partials(c->kpart.p, round_up(n, kPad), c->kplan.nslots, n, acc, nullptr,
                                           (flags & KHRR_OVERWRITE) != 0, c->stream),
                    "reduce partials");
@@ -254,6 +259,10 @@ khrr_status khrr_phi(khrr_ctx* c, double* phi, const double* pos_i, const double
         return c->cuda(launch_reduce_pair_fx(c->kfx.p, round_up(n, kPad), c->kscale.p, n, nullptr, phi,
                                              (flags & KHRR_OVERWRITE) != 0, c->stream),
                        "reduce sums");
+    if (c->kplan.chains > 0)
+        return c->cuda(launch_reduce_tiles(reinterpret_cast<const float4*>(c->kpart.p), round_up(n, kPad), c->kplan.ntiles,
+                                           c->kplan.chains, n, nullptr, phi, (flags & KHRR_OVERWRITE) != 0, c->stream),
+                       "reduce partials");
     return c->cuda(launch_reduce_partials(c->kpart.p, round_up(n, kPad), c->kplan.nslots, n, nullptr, phi,
                                           (flags & KHRR_OVERWRITE) != 0, c->stream),
                    "reduce partials");

@@ -51,11 +51,16 @@ struct ForceArgs {
     int n_items;
     unsigned* queue;         // next-item counter (zeroed before each launch)
     double4* part;           // partial sums [slot][npad]: ax, ay, az, sum m/r
+    float4* tiles;           // when set, every j tile's FP32 partials [tile][npad] instead (without the factored mass)
     long long npad;          // slot stride
     float h_uniform;         // 0.5 * eps2 when every body shares it
     const float* tile_mass;  // mass of each 128-body j tile (tile-mass kernels only)
     unsigned* err;           // device error flag word
 };
+
+// acc[i] (+)= a_i and/or phi[i] (-)= sum m/r from the tiles' partials.
+cudaError_t launch_reduce_tiles(const float4* tiles, long long npad, int ntiles, int chains, int64_t n, double* acc,
+                                double* phi, bool overwrite, cudaStream_t s);
 
 // One compiled force-kernel instance.  pair: the symmetric kernel (pair.cu),
 // launched with PairArgs; its tile_mass means one mass per kPairBlock block.
@@ -234,6 +239,9 @@ struct StepArgs {
     const double4* part;  // force partials [slot][npad]
     long long npad;
     const unsigned char* nsplit;  // partial slots per body
+    const float4* tiles;          // the one-sided kernel's partials per j tile [ntiles][npad] (replace part when set)
+    int ntiles, chains;           // ... summed in this many runs
+    const float* tile_mass;       // ... and their factored masses (null: none)
     unsigned long long* fx;         // the pair kernel's fixed-point sums [kFxComps][npad] (replace part when set)
     const FxScale* fx_scale;        // their scales per 128-body tile
     double* f64;          // the symmetric FP64 pass's sums [2][4][npad] (replace part when set)

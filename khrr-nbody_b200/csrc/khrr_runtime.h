@@ -60,6 +60,11 @@ struct ForcePlan {
     std::vector<WorkItem> items;
     std::vector<int> sys_item_begin;  // plain plans: items of system k
     std::vector<int> sys_split;       // j chunks per system
+    int chains = 0, ntiles = 0;       // > 0: items leave one partial per j tile, summed in this many runs
+    // double4 words of the partials of npad bodies
+    size_t partial_words(int64_t npad) const {
+        return static_cast<size_t>(chains > 0 ? (ntiles + 1) / 2 : nslots) * static_cast<size_t>(npad);
+    }
     int nslots = 1;
     DevBuf<WorkItem> d_items;
     DevBuf<unsigned char> d_nsplit;

@@ -3,22 +3,10 @@
 
 #include <cstdint>
 
+#include "tile_sums.cuh"
+
 namespace khrr {
 namespace {
-
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-__device__ __forceinline__ void two_sum_into(float& hi, float& lo, float p) {
-    const float s = hi + p;
-    const float bp = s - hi;
-    const float e = (hi - (s - bp)) + (p - bp);
-    hi = s;
-    lo += e;
-}
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
