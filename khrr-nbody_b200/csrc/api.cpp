@@ -19,6 +19,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -34,6 +35,48 @@ using namespace khrr;
 // helpers
 // ---------------------------------------------------------------------------
 namespace {
+
+// Page-locked words for contexts, kHostWords doubles each.  Allocating and
+// freeing page-locked memory takes 2 ms or more, a context's creation without
+// it 3 ms: the slots of one page, kept for the process, serve up to 16 contexts
+// at a time, and any more allocate their own.
+constexpr size_t kHostWords = 32, kHostSlots = 16;
+std::mutex host_page_mutex;
+double* host_page = nullptr;
+unsigned host_page_used = 0;  // one bit per slot
+
+cudaError_t take_host_words(double** out) {
+    std::lock_guard<std::mutex> lock(host_page_mutex);
+    cudaPointerAttributes at{};
+    if (host_page && (cudaPointerGetAttributes(&at, host_page) != cudaSuccess || at.type != cudaMemoryTypeHost)) {
+        (void)cudaGetLastError();  // the program reset its device: the page is gone
+        host_page = nullptr;
+        host_page_used = 0;
+    }
+    if (!host_page) {
+        const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&host_page),
+                                            kHostSlots * kHostWords * sizeof(double), cudaHostAllocPortable);
+        if (e != cudaSuccess) {
+            host_page = nullptr;
+            return e;
+        }
+    }
+    for (size_t k = 0; k < kHostSlots; ++k)
+        if (!(host_page_used >> k & 1u)) {
+            host_page_used |= 1u << k;
+            *out = host_page + k * kHostWords;
+            return cudaSuccess;
+        }
+    return cudaHostAlloc(reinterpret_cast<void**>(out), kHostWords * sizeof(double), cudaHostAllocPortable);
+}
+
+// After the context's last work on its stream has ended.
+void give_host_words(double* p) {
+    std::lock_guard<std::mutex> lock(host_page_mutex);
+    if (host_page && p >= host_page && p < host_page + kHostSlots * kHostWords)
+        host_page_used &= ~(1u << ((p - host_page) / kHostWords));
+    else cudaFreeHost(p);
+}
 
 int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
@@ -916,7 +959,7 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
         c->queue.ensure(kQueueWords) != cudaSuccess || c->errflag.ensure(1) != cudaSuccess ||
         c->cons_done.ensure(1) != cudaSuccess ||
         c->scratch.ensure(64) != cudaSuccess ||
-        cudaHostAlloc(reinterpret_cast<void**>(&c->host_words), 17 * sizeof(double), cudaHostAllocDefault) != cudaSuccess) {
+        take_host_words(&c->host_words) != cudaSuccess) {
         khrr_destroy(c);
         return KHRR_ERR_CUDA;
     }
@@ -955,8 +998,9 @@ void khrr_destroy(khrr_ctx* c) {
     if (c->ph0) cudaEventDestroy(c->ph0);
     if (c->ph1) cudaEventDestroy(c->ph1);
     if (c->own) cudaStreamDestroy(c->own);
-    if (c->host_words) cudaFreeHost(c->host_words);
-    delete c;  // device buffers free themselves
+    double* words = c->host_words;
+    delete c;  // device buffers free themselves, after the device's work
+    if (words) give_host_words(words);
 }
 
 const char* khrr_last_error(const khrr_ctx* c) { return c ? c->err.c_str() : "null context"; }
