@@ -308,7 +308,7 @@ cudaError_t launch_scan(int* count, bool pair, int64_t ncells, int* maxpbc, int*
 cudaError_t launch_cell_phi(const double* phi, const int2* pci, const int* count, int cstride, int64_t n,
                             double* cell_phi, cudaStream_t s);
 cudaError_t launch_wave_f64(double* phi_new, const double* phi, const double* phi_old, const double* mass,
-                            const WaveConsts& w, cudaStream_t s);
+                            const WaveConsts& w, unsigned* err, cudaStream_t s);
 cudaError_t launch_wave_f32(float* phi_new, const float* phi, const float* phi_old, const float* mass,
                             const WaveF32& w, double* resid, cudaStream_t s);
 // The four-buffer field ring of the FP32 solver: state = 4 * old + cur; a

@@ -29,7 +29,7 @@
 #include "async_copy.cuh"
 #include "khrr_internal.h"
 #include "wave_bricks.h"
-#include "wave_march.cuh"
+#include "wave_stream.cuh"
 
 namespace khrr {
 namespace {
@@ -1311,15 +1311,30 @@ cudaError_t launch_cell_phi(const double* phi, const int2* pci, const int* count
 }
 
 cudaError_t launch_wave_f64(double* phi_new, const double* phi, const double* phi_old, const double* mass,
-                            const WaveConsts& w, cudaStream_t s) {
+                            const WaveConsts& w, unsigned* err, cudaStream_t s) {
     // Pairs of cells where the rows and the caller's arrays allow 16-byte
-    // accesses.  us per iteration at 64^3 / 100^3 / 128^3 / 200^3 / 256^3: 3.2 /
+    // accesses.  The march, us per iteration at 64^3 / 100^3 / 128^3 / 200^3 / 256^3: 3.2 /
     // 6.8 / 12.2 / 54.7 / 108.9 (one cell per thread and launch of 249
     // instructions a cell: 6.2 / 14.5 / 20.6 / 82.5 / 153.5); 128 threads, five
     // blocks per SM; 256 x 2 2.8 / 7.1 / 12.0 / 60.6 / 120.3, six blocks spill
     // (75.7 at 200^3).  Single cells (201^3): 64.6 against 84.5.
     const uintptr_t any = reinterpret_cast<uintptr_t>(phi_new) | reinterpret_cast<uintptr_t>(phi) |
                           reinterpret_cast<uintptr_t>(phi_old) | reinterpret_cast<uintptr_t>(mass);
+    if (w.nx % 2 == 0 && any % 16 == 0 && w.nx >= 178 && w.nx <= 352) {
+        // The planes through shared memory where the field does not stay in L2:
+        // us per iteration, march / this, 33.6 / 30.9 at 170^3, 35.1 / 36.8 at
+        // 176^3, 39.4 / 35.1 at 180^3, 51.7 / 45.6 at 200^3, 255.8 / 217.1 at
+        // 350^3, 275.2 / 279.5 at 360^3, 382.3 / 382.7 at 400^3.
+        // Segments of 1,280 cells and three stages, or of 1,024 and four: the one
+        // whose blocks fill the chip better (us per iteration, 1,280 / 1,024:
+        // 45.3 / 46.0 at 200^3, 62.7 / 58.9 at 220^3, 75.3 / 73.8 at 240^3, 91.2 /
+        // 97.9 at 256^3, 180 / 229 at 320^3).
+        using Wide = StreamShape<320, 2, 2, 3>;
+        using Deep = StreamShape<256, 2, 2, 4>;
+        const StreamCut wide = Wide::cut(w.nx), deep = Deep::cut(w.nx);
+        return wide.cost <= deep.cost ? Wide::launch(wide, phi_new, phi, phi_old, mass, w, err, s)
+                                      : Deep::launch(deep, phi_new, phi, phi_old, mass, w, err, s);
+    }
     if (w.nx % 2 == 0 && any % 16 == 0)
         return launch_march<StepF64<2>, 2, 128, 5, false>(phi_new, phi, phi_old, mass, w, w.nx, nullptr, s);
     return launch_march<StepF64<1>, 1, 256, 4, false>(phi_new, phi, phi_old, mass, w, w.nx, nullptr, s);

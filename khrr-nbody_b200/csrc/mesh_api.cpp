@@ -206,7 +206,8 @@ khrr_status khrr_wave_iteration(khrr_ctx* c, double* phi_new, const double* phi,
     khrr_status st = check_wave(c, p);
     if (st != KHRR_OK) return st;
     if (!phi_new || !phi || !phi_old || !cell_mass) return c->fail(KHRR_ERR_INVALID_ARG, "null mesh array");
-    return c->cuda(launch_wave_f64(phi_new, phi, phi_old, cell_mass, wave_consts(p), c->stream), "wave iteration");
+    return c->cuda(launch_wave_f64(phi_new, phi, phi_old, cell_mass, wave_consts(p), c->errflag.p, c->stream),
+                   "wave iteration");
 }
 
 khrr_status khrr_acc_field(khrr_ctx* c, double* cell_acc, double* cell_acc_abs, const double* cell_phi, int nx,
@@ -692,7 +693,7 @@ khrr_status khrr_ctx::mesh_enqueue_force(const double* x, int iters, int rot0) {
             double* old = M.phi64.p + static_cast<size_t>(r / 4) * cz;
             double* cur = M.phi64.p + static_cast<size_t>(r % 4) * cz;
             double* nxt = M.phi64.p + static_cast<size_t>(f0) * cz;
-            if ((st = cuda(launch_wave_f64(nxt, cur, old, M.cell_mass.p, w, s), "wave")) != KHRR_OK) return st;
+            if ((st = cuda(launch_wave_f64(nxt, cur, old, M.cell_mass.p, w, errflag.p, s), "wave")) != KHRR_OK) return st;
         }
         const double* cur = M.phi64.p + static_cast<size_t>(r % 4) * cz;
         if ((st = cuda(launch_acc_field(M.cell_acc.p, nullptr, cur, nx, P.wave.dx, s), "acc_field")) != KHRR_OK)

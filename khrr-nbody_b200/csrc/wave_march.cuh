@@ -102,7 +102,7 @@ struct StepF32 {
 template <int V>
 struct StepF64 {
     using T = double;
-    const WaveConsts W;
+    WaveConsts W;
     double L, D3, yD3, K, KFn, KAn;
     double sxy[V], km[V], ka[V], ko[V], kf[V];
     __device__ __forceinline__ double term(double p, bool above, bool below) const {
