@@ -151,13 +151,13 @@ __global__ void __launch_bounds__(NT, kMinCtas) fp64_force_kernel(const F64Args 
 //
 // The kernel is bound by the FP64 pipe (64 lanes per SM and clock), so what
 // counts is FP64 instructions per unordered pair:
-//   * r^-1 and r^-3 from the hardware's reciprocal-square-root seed y0 (one
-//     XU instruction on the upper word, relative error 2^-20) and the
-//     binomial series of (1 - e)^(-1/2) and (1 - e)^(-3/2) in e = 1 - r2 y0^2
-//     (y0^2 is exact, y0 having 21 significant bits), cut after e^2: the
-//     terms left out are 5/16 e^3 and 35/16 e^3, below 2^-55 for |e| < 2^-19.  Six operations for r^-3 (five for r^-1 and two more for
-//     its cube when the potential is wanted too) instead of rsqrt() with its
-//     range handling and two multiplies.
+//   * r^-3 from the hardware's reciprocal-square-root seed y0 (one XU
+//     instruction on the upper word, relative error 2^-20) and the binomial
+//     series of (1 - e)^(-3/2) in e = 1 - r2 y0^2 (y0^2 is exact, y0 having 21
+//     significant bits), cut after e^2: the term left out is 35/16 e^3, below
+//     2^-55 for |e| < 2^-19.  Six operations, and r^-1 = r2 r^-3 where the
+//     potential is wanted too, instead of rsqrt() with its range handling and
+//     two multiplies.
 //   * where the i block has one mass and one softening and so has the j tile
 //     (all but the tiles at a component's border and a ragged end), the
 //     masses leave the pair term (applied once per sum) and h_i + h_j is a
@@ -203,13 +203,9 @@ __device__ __forceinline__ void inverse_powers(double r2, double& inv, double& i
     const double y0 = rsqrt_seed(r2);
     const double s = y0 * y0;
     const double e = fma(-r2, s, 1.0);
-    if (PHI) {
-        inv = fma(y0 * e, fma(0.375, e, 0.5), y0);
-        i3 = inv * inv * inv;
-    } else {
-        const double c = s * y0;
-        i3 = fma(c * e, fma(1.875, e, 1.5), c);
-    }
+    const double c = s * y0;
+    i3 = fma(c * e, fma(1.875, e, 1.5), c);
+    if (PHI) inv = r2 * i3;
 }
 
 // Adds v into the pair of sums, cut at the grid 2^-52 c / 1.5.
