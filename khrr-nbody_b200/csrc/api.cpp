@@ -956,8 +956,8 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
     c->sm_count = prop.multiProcessorCount;
     if (cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ph0) != cudaSuccess || cudaEventCreate(&c->ph1) != cudaSuccess ||
-        c->queue.ensure(kQueueWords) != cudaSuccess || c->errflag.ensure(1) != cudaSuccess ||
-        c->cons_done.ensure(1) != cudaSuccess ||
+        c->queue.ensure(kQueueWords) != cudaSuccess || c->kqueue.ensure(kQueueWords) != cudaSuccess ||
+        c->errflag.ensure(1) != cudaSuccess || c->cons_done.ensure(1) != cudaSuccess ||
         c->scratch.ensure(64) != cudaSuccess ||
         take_host_words(&c->host_words) != cudaSuccess) {
         khrr_destroy(c);

@@ -155,14 +155,13 @@ khrr_status prepare_kernel_pass(khrr_ctx* c, const double* pos_i, const double* 
 
 khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i) {
     ForcePlan& p = c->kplan;
-    c->clean = 0;  // the state's force passes share the queue counter
     const int64_t npad = round_up(c->kplan_n, kPad);
     if (v->pair) {
         PairArgs a{};
         a.sh = shadow_at(c->kshadow.p, npad);
         a.items = p.d_pair_items.p;
         a.n_items = static_cast<int>(p.pair_items.size());
-        a.queue = c->queue.p;
+        a.queue = c->kqueue.p;
         a.share = p.pair_share;
         a.fx = c->kfx.p;
         a.npad = npad;
@@ -174,7 +173,8 @@ khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i)
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         khrr_status st;
         if (c->timing && (st = c->timing_pair(&e0, &e1)) != KHRR_OK) return st;
-        if ((st = c->cuda(cudaMemsetAsync(c->queue.p, 0, kQueueWords * sizeof(unsigned), s), "queue reset")) != KHRR_OK) return st;
+        if ((st = c->cuda(cudaMemsetAsync(c->kqueue.p, 0, kQueueWords * sizeof(unsigned), s), "queue reset")) != KHRR_OK)
+            return st;
         if ((st = c->cuda(cudaMemsetAsync(c->kfx.p, 0, sizeof(unsigned long long) * kFxComps * npad, s),
                           "sums reset")) != KHRR_OK)
             return st;
@@ -196,7 +196,7 @@ khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i)
     a.i = distinct_i ? shadow_at(c->kishadow.p, npad) : a.j;
     a.items = p.d_items.p;
     a.n_items = static_cast<int>(p.items.size());
-    a.queue = c->queue.p;
+    a.queue = c->kqueue.p;
     a.part = c->kpart.p;
     a.tiles = p.chains > 0 ? reinterpret_cast<float4*>(c->kpart.p) : nullptr;
     a.npad = npad;
@@ -206,7 +206,7 @@ khrr_status run_kernel_pass(khrr_ctx* c, const ForceVariant* v, bool distinct_i)
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     khrr_status st;
     if (c->timing && (st = c->timing_pair(&e0, &e1)) != KHRR_OK) return st;
-    if ((st = c->cuda(cudaMemsetAsync(c->queue.p, 0, sizeof(unsigned), s), "queue reset")) != KHRR_OK) return st;
+    if ((st = c->cuda(cudaMemsetAsync(c->kqueue.p, 0, sizeof(unsigned), s), "queue reset")) != KHRR_OK) return st;
     if (e0) cudaEventRecord(e0, s);
     const int grid = std::min(a.n_items, c->resident_ctas(v));
     if ((st = c->cuda(launch_force(v, a, grid, s), "force kernel")) != KHRR_OK) return st;

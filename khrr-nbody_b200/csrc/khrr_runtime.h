@@ -197,7 +197,10 @@ struct khrr_ctx {
     int clean = 0;
     khrr_status ensure_clean(int mode);
 
-    // Kernel-level entry points: their own shadow, partials and plan.
+    // Kernel-level entry points: their own shadow, partials, plan and queue
+    // words (a graph of the caller's may replay such a pass between the state's
+    // passes, whose own words `clean` describes).
+    khrr::DevBuf<unsigned> kqueue;
     khrr::DevBuf<float> kshadow, kishadow;
     khrr::DevBuf<double4> kpart;
     khrr::DevBuf<unsigned long long> kfx;  // the pair kernel's sums (pos_i == pos_j under the pair tuning)
