@@ -58,6 +58,14 @@ constexpr unsigned kAcc = 2;      // accumulate accelerations
 constexpr unsigned kPhi = 4;      // accumulate potentials
 constexpr unsigned kPacked = 8;   // packed f32x2 inner loop (two j bodies per instruction)
 constexpr unsigned kTileMass = 16;  // each j tile has one mass (ForceArgs::tile_mass): m factored out
+// A few thousand bodies: one partial per j tile and body (ForceArgs::tiles)
+// instead of the items' sums, which the reader forms.  A kernel of its own: as
+// a branch of the others it cost them two to eight registers, which took a CTA
+// per SM from the potential-only ones and changed the order of the others' loop
+// (us per pass with the branch / without it: potential 316 / 267 at 30,720
+// bodies and 1115 / 1003 at 61,440; at 49,152, one mass per tile, acceleration
+// 1015 / 963, with the potential 1047 / 994).
+constexpr unsigned kTiles = 32;
 
 template <int NT, int K, int JT, int STAGES, unsigned F>
 struct ForceShape {
@@ -113,9 +121,9 @@ constexpr int force_min_blocks() {
 
 template <int NT, int K, int JT, int STAGES, unsigned F>
 __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kernel(const ForceArgs a) {
-    using S = ForceShape<NT, K, JT, STAGES, F>;
+    using S = ForceShape<NT, K, JT, STAGES, F & ~kTiles>;
     constexpr bool UNIF = S::UNIF, ACC = S::ACC, PHI = S::PHI, TMASS = S::TMASS;
-    constexpr bool PACKED = F & kPacked;
+    constexpr bool PACKED = F & kPacked, TILES = F & kTiles;
     constexpr int NC = S::NC;
     constexpr int NCOMP = S::NCOMP;
     static_assert(NC > 0, "nothing to accumulate");
@@ -152,12 +160,16 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
     // With no more items than CTAs every CTA takes its own and nothing waits for
     // the queue (two round trips to L2 in a pass of a few microseconds: with
     // the corrector's loads ahead 14.3 -> 12.3 us per time step of 3,072
-    // bodies).  A first item without the queue for any number of items changed
-    // the compiled loop as well: 1483 -> 1613 us per step of 61,440 bodies with
-    // two softenings.
+    // bodies).  The test for it changes the compiled loop as well, for the
+    // better or the worse: only the kernel of the small systems and the general
+    // packed one of the default shape have it (us per pass with it / without:
+    // masses and softenings per body, acceleration and potential, 7984 / 8218
+    // at 131,072 bodies, 1213 / 1260 at 49,152; one softening, one mass per
+    // tile, 1061 / 994 at 49,152 and potential alone 1112 / 1003 at 61,440).
+    constexpr bool OWN_FIRST = TILES || (PACKED && ACC && !UNIF && !TMASS && NT == 128 && K == 4);
     for (;;) {
         if (tid == 0) {
-            if (a.n_items > static_cast<int>(gridDim.x)) s_item = static_cast<int>(atomicAdd(a.queue, 1u));
+            if (!OWN_FIRST || a.n_items > static_cast<int>(gridDim.x)) s_item = static_cast<int>(atomicAdd(a.queue, 1u));
             else s_item = consumed == 0u ? static_cast<int>(blockIdx.x) : a.n_items;
         }
         __syncthreads();
@@ -264,7 +276,7 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
                     }
                 }
             }
-            if (a.tiles) {
+            if (TILES) {
                 // A few thousand bodies: the runs of tiles that one item sums
                 // below are shared by several, and the reader sums them.
                 float4* out = a.tiles + ((w.j_begin - a.items[0].j_begin) / JT + t) * a.npad;
@@ -309,11 +321,12 @@ __global__ void __launch_bounds__(NT, (force_min_blocks<NT, K, F>())) force_kern
         }
         consumed += static_cast<unsigned>(ntiles);
 
+        if (TILES) continue;  // the partials are written; a.part holds them, not slots
         double4* out = a.part + static_cast<long long>(w.slot) * a.npad;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int i = w.i_begin + k * NT + tid;
-            if (i < w.i_end && !a.tiles) {
+            if (i < w.i_end) {
                 double4 o;
                 o.x = o.y = o.z = o.w = 0.0;
                 int c = 0;
@@ -344,7 +357,8 @@ ForceVariant make_variant() {
                         (F & kPhi) != 0,
                         (F & kTileMass) != 0,
                         reinterpret_cast<const void*>(&force_kernel<NT, K, JT, STAGES, F>),
-                        S::kSmem};
+                        S::kSmem,
+                        reinterpret_cast<const void*>(&force_kernel<NT, K, JT, STAGES, F | kTiles>)};
 }
 
 // Every softening form x every output set of one shape (and mass form).
@@ -601,7 +615,7 @@ const ForceVariant* find_force_variant(int threads, int ipt, int jt, bool packed
 cudaError_t launch_force(const ForceVariant* v, const ForceArgs& a, int grid, cudaStream_t s) {
     ForceArgs args = a;
     void* params[] = {&args};
-    return cudaLaunchKernel(v->fn, dim3(grid), dim3(v->threads), params, v->smem, s);
+    return cudaLaunchKernel(a.tiles ? v->fn_tiles : v->fn, dim3(grid), dim3(v->threads), params, v->smem, s);
 }
 
 cudaError_t launch_plain_force(const Shadow& sh, int n, int npad, double4* out, bool acc, bool phi,

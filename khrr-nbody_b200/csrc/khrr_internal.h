@@ -69,6 +69,7 @@ struct ForceVariant {
     bool packed, uniform_eps, acc, phi, tile_mass;
     const void* fn;
     size_t smem;
+    const void* fn_tiles = nullptr;  // the one-sided kernel that leaves a partial per tile (ForceArgs::tiles)
     bool pair = false;
 };
 
