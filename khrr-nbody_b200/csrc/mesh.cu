@@ -1151,15 +1151,15 @@ __global__ void __launch_bounds__(256) cic_combine_kernel(double* __restrict__ c
 }
 
 // Interpolation back to a body by its two lanes (a: the lane's x corner): acc
-// (3 per cell) and a scalar field in FP32 or FP64.  The products of the second
-// corner reach the first lane by shuffle and the sums run in z, y, x corner
-// order there, as one thread would form them; corners outside the mesh add
+// (3 per cell) and a scalar field in FP32 or FP64 (VAL).  The first lane ends
+// with acc x and y in s, the second with acc z and the value: each hands the
+// other its corner's products of the other's two sums, which run in z, y, x
+// corner order, as one thread would form them; corners outside the mesh add
 // nothing.  Every lane of the warp takes part (p: any address in bounds for
-// lanes past the bodies).  The result is the first lane's.
-template <class T>
+// lanes past the bodies).
+template <bool VAL, class T>
 __device__ __forceinline__ void cic_interp(const double* __restrict__ p, int a, const MeshGeom& m,
-                                           const double* __restrict__ cacc, const T* __restrict__ cval, double (&acc)[3],
-                                           double& val) {
+                                           const double* __restrict__ cacc, const T* __restrict__ cval, double (&s)[2]) {
     const CicAxis ax = cic_axis(p[0], m.lo[0], m.cs[0], m.rcs[0], m.g[0]);
     const CicAxis ay = cic_axis(p[1], m.lo[1], m.cs[1], m.rcs[1], m.g[1]);
     const CicAxis az = cic_axis(p[2], m.lo[2], m.cs[2], m.rcs[2], m.g[2]);
@@ -1167,8 +1167,7 @@ __device__ __forceinline__ void cic_interp(const double* __restrict__ p, int a, 
     const bool x_in = x >= 0 && x < m.g[0];
     const bool x0_in = ax.i0 >= 0 && ax.i0 < m.g[0], x1_in = ax.i0 + 1 >= 0 && ax.i0 + 1 < m.g[0];
     const double wx = a ? ax.w[1] : ax.w[0];
-    acc[0] = acc[1] = acc[2] = 0.0;
-    val = 0.0;
+    s[0] = s[1] = 0.0;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int z = az.i0 + c;
@@ -1180,39 +1179,73 @@ __device__ __forceinline__ void cic_interp(const double* __restrict__ p, int a, 
             if (row_in && x_in) {
                 const double w = (wx * ay.w[b]) * az.w[c];
                 const int64_t id = static_cast<int64_t>(z) * m.g[0] * m.g[1] + static_cast<int64_t>(y) * m.g[2] + x;
-                if (cacc) {
-                    q[0] = w * cacc[3 * id];
-                    q[1] = w * cacc[3 * id + 1];
-                    q[2] = w * cacc[3 * id + 2];
-                }
-                if (cval) q[3] = w * static_cast<double>(cval[id]);
+                q[0] = w * cacc[3 * id];
+                q[1] = w * cacc[3 * id + 1];
+                q[2] = w * cacc[3 * id + 2];
+                if (VAL) q[3] = w * static_cast<double>(cval[id]);
             }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                if (k < 3 ? !cacc : !cval) continue;
-                const double second = __shfl_down_sync(0xffffffffu, q[k], 1);
-                double& sum = k < 3 ? acc[k] : val;
-                if (row_in && x0_in) sum += q[k];
-                if (row_in && x1_in) sum += second;
+            for (int k = 0; k < 2; ++k) {
+                const double other = __shfl_xor_sync(0xffffffffu, a ? q[k] : q[2 + k], 1);
+                const double first = a ? other : q[k], second = a ? q[2 + k] : other;
+                if (row_in && x0_in) s[k] += first;
+                if (row_in && x1_in) s[k] += second;
             }
         }
     }
 }
 
+// Two lanes per body where the accelerations are wanted, against one (us, one ->
+// two): evenly spread bodies, with the value, 70 -> 44 at 786,432 on 64^3,
+// 501 -> 325 for 2 M on 256^3; a galaxy, whose neighbours in memory are close
+// in space, 38 -> 36 and 138 -> 103.
+template <bool VAL>
 __global__ void __launch_bounds__(256) cic_gather_kernel(const double* __restrict__ pos, int64_t n, const MeshGeom m,
                                                          const double* __restrict__ cacc,
                                                          const double* __restrict__ cval, double* __restrict__ pacc,
                                                          double* __restrict__ pval) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, i = t >> 1;
-    double a[3], v;
-    cic_interp(pos + 3 * min(i, n - 1), static_cast<int>(t & 1), m, pacc ? cacc : nullptr, pval ? cval : nullptr, a, v);
-    if (i >= n || (t & 1)) return;
-    if (pacc) {
-        pacc[3 * i] = a[0];
-        pacc[3 * i + 1] = a[1];
-        pacc[3 * i + 2] = a[2];
+    double s[2];
+    cic_interp<VAL>(pos + 3 * min(i, n - 1), static_cast<int>(t & 1), m, cacc, cval, s);
+    if (i >= n) return;
+    if (t & 1) {
+        pacc[3 * i + 2] = s[0];
+        if (VAL) pval[i] = s[1];
+    } else {
+        pacc[3 * i] = s[0];
+        pacc[3 * i + 1] = s[1];
     }
-    if (pval) pval[i] = v;
+}
+
+// The value alone, one lane per body: 8 bytes a corner give two lanes too little
+// to share (us, two lanes -> one: a galaxy of 786,432 on 64^3 25.3 -> 15.1, 2 M
+// on 128^3 56.1 -> 29.3, evenly spread 60.4 -> 46.3).
+__global__ void __launch_bounds__(256) cic_value_kernel(const double* __restrict__ pos, int64_t n, const MeshGeom m,
+                                                        const double* __restrict__ cval, double* __restrict__ pval) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const CicAxis ax = cic_axis(pos[3 * i], m.lo[0], m.cs[0], m.rcs[0], m.g[0]);
+    const CicAxis ay = cic_axis(pos[3 * i + 1], m.lo[1], m.cs[1], m.rcs[1], m.g[1]);
+    const CicAxis az = cic_axis(pos[3 * i + 2], m.lo[2], m.cs[2], m.rcs[2], m.g[2]);
+    double val = 0.0;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int z = az.i0 + c;
+        if (z < 0 || z >= m.g[2]) continue;
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int y = ay.i0 + b;
+            if (y < 0 || y >= m.g[1]) continue;
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                const int x = ax.i0 + a;
+                if (x < 0 || x >= m.g[0]) continue;
+                const int64_t id = static_cast<int64_t>(z) * m.g[0] * m.g[1] + static_cast<int64_t>(y) * m.g[2] + x;
+                val += ((ax.w[a] * ay.w[b]) * az.w[c]) * cval[id];
+            }
+        }
+    }
+    pval[i] = val;
 }
 
 // The mesh-force gather into the corrector's partial slot: {acc, -phi}, so
@@ -1223,9 +1256,10 @@ __global__ void __launch_bounds__(256) mesh_gather_cic_kernel(const double* __re
                                                               const MeshGeom m, const double* __restrict__ cacc,
                                                               const T* __restrict__ phi, double4* __restrict__ part) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, i = t >> 1;
-    double a[3], v;
-    cic_interp(pos + 3 * min(i, n - 1), static_cast<int>(t & 1), m, cacc, phi, a, v);
-    if (i < n && !(t & 1)) part[i] = make_double4(a[0], a[1], a[2], -v);
+    const int a = static_cast<int>(t & 1);
+    double s[2];
+    cic_interp<true>(pos + 3 * min(i, n - 1), a, m, cacc, phi, s);
+    if (i < n) reinterpret_cast<double2*>(part + i)[a] = make_double2(s[0], a ? -s[1] : s[1]);
 }
 
 template <class T>
@@ -1519,8 +1553,15 @@ cudaError_t launch_cic_deposit(const double* pos, const double* mass, int64_t n,
 cudaError_t launch_cic_gather(const double* pos, int64_t n, const MeshGeom& m, const double* cell_acc,
                               const double* cell_value, double* pacc, double* pval, cudaStream_t s) {
     if (n < 1) return cudaSuccess;
-    cic_gather_kernel<<<static_cast<unsigned>((2 * n + 255) / 256), 256, 0, s>>>(pos, n, m, cell_acc, cell_value, pacc,
-                                                                                   pval);
+    if (!pacc && !pval) return cudaSuccess;
+    if (!pacc)
+        cic_value_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(pos, n, m, cell_value, pval);
+    else if (pval)
+        cic_gather_kernel<true><<<static_cast<unsigned>((2 * n + 255) / 256), 256, 0, s>>>(pos, n, m, cell_acc, cell_value,
+                                                                                           pacc, pval);
+    else
+        cic_gather_kernel<false><<<static_cast<unsigned>((2 * n + 255) / 256), 256, 0, s>>>(pos, n, m, cell_acc, nullptr,
+                                                                                            pacc, nullptr);
     return cudaGetLastError();
 }
 
