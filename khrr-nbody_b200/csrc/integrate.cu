@@ -15,6 +15,7 @@
 // in IEEE double.
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 #include "khrr_internal.h"
 #include "tile_sums.cuh"
@@ -105,15 +106,24 @@ __global__ void predictor_kernel(const StepArgs a) {
     }
 }
 
+// Where a pass left its sums: the pair kernel's fixed-point words, the symmetric
+// FP64 pass's two parts, the one-sided kernel's partial per tile, or its slots.
+// The kernels that read them are compiled for each: in one kernel the partials'
+// loads ahead set the registers of all (214, one block per SM where there were
+// four), and the corrector of 393,216 bodies with one slot took 31.5 us where it takes 18.7
+// now, a collect 21.8 and 7.0.
+enum class Src { kFx, kF64, kTiles, kSlots, kFewSlots };
+
 // The sums of body i; the accumulating kernels' (fx, f64) are left zero for
 // the next pass, and so is its queue: two memsets less per step (about 2 us
 // each between small kernels).
+template <Src S>
 __device__ __forceinline__ void sum_partials(const StepArgs& a, int64_t i, d3& s, double& sp) {
     s = d3{0.0, 0.0, 0.0};
     sp = 0.0;
     if (a.queue)
         for (int64_t q = i; q < kQueueWords; q += a.n) a.queue[q] = 0u;
-    if (a.fx) {
+    if constexpr (S == Src::kFx) {
         // The pair kernel's fixed-point sums (zero for ghosts).
         const FxScale sc = a.fx_scale[i / kPad];
         s.x = static_cast<double>(static_cast<long long>(a.fx[i])) * sc.inv_acc;
@@ -122,50 +132,48 @@ __device__ __forceinline__ void sum_partials(const StepArgs& a, int64_t i, d3& s
         sp = static_cast<double>(static_cast<long long>(a.fx[3 * a.npad + i])) * sc.inv_phi;
 #pragma unroll
         for (int c = 0; c < kFxComps; ++c) a.fx[c * a.npad + i] = 0ull;
-        return;
-    }
-    if (a.f64) {
+    } else if constexpr (S == Src::kF64) {
         double *u = a.f64 + i, *l = u + 4 * a.npad;
         s = d3{u[0] + l[0], u[a.npad] + l[a.npad], u[2 * a.npad] + l[2 * a.npad]};
         sp = u[3 * a.npad] + l[3 * a.npad];
 #pragma unroll
         for (int c = 0; c < 8; ++c) u[c * a.npad] = 0.0;
-        return;
-    }
-    if (a.tiles) {
+    } else if constexpr (S == Src::kTiles) {
         if (a.nsplit[i] == 0) return;
         const double4 t = sum_tile_chains<16>(a.tiles, a.npad, i, a.ntiles, a.chains, a.tile_mass);
         s = d3{t.x, t.y, t.z};
         sp = t.w;
-        return;
-    }
-    // Slots in order, eight loads in flight (a small system's 24 slots one
-    // after the other took most of the corrector's 8 us).
-    const int ns = a.nsplit[i];
-    constexpr int kAhead = 8;
-    for (int k0 = 0; k0 < ns; k0 += kAhead) {
-        double4 p[kAhead];
+    } else {
+        // Slots in order, eight loads in flight where the bodies are few (a
+        // small system's 24 slots one after the other took most of the
+        // corrector's 8 us) and the other warps cannot cover them.
+        const int ns = a.nsplit[i];
+        constexpr int kAhead = S == Src::kFewSlots ? 8 : 1;
+        for (int k0 = 0; k0 < ns; k0 += kAhead) {
+            double4 p[kAhead];
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k)
-            if (k0 + k < ns) p[k] = a.part[(k0 + k) * a.npad + i];
+            for (int k = 0; k < kAhead; ++k)
+                if (k0 + k < ns) p[k] = a.part[(k0 + k) * a.npad + i];
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k)
-            if (k0 + k < ns) {
-                s.x += p[k].x;
-                s.y += p[k].y;
-                s.z += p[k].z;
-                sp += p[k].w;
-            }
+            for (int k = 0; k < kAhead; ++k)
+                if (k0 + k < ns) {
+                    s.x += p[k].x;
+                    s.y += p[k].y;
+                    s.z += p[k].z;
+                    sp += p[k].w;
+                }
+        }
     }
 }
 
 // Corrector (istep 1) fused with the next predictor.
+template <Src S>
 __global__ void corrector_kernel(const StepArgs a) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
          i += (int64_t)gridDim.x * blockDim.x) {
         d3 an;
         double sp;
-        sum_partials(a, i, an, sp);
+        sum_partials<S>(a, i, an, sp);
         if (a.compat_accumulate) {
             // The reference adds each step's force onto acct_ (never zeroed).
             d3 prev = ld3(a.acct, i);
@@ -188,12 +196,13 @@ __global__ void corrector_kernel(const StepArgs a) {
 }
 
 // Partials -> state acc/phi (khrr_forces).
+template <Src S>
 __global__ void collect_kernel(const StepArgs a, int want_acc, int accumulate) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
          i += (int64_t)gridDim.x * blockDim.x) {
         d3 s;
         double sp;
-        sum_partials(a, i, s, sp);
+        sum_partials<S>(a, i, s, sp);
         if (want_acc) {
             if (accumulate) {
                 const d3 prev = ld3(a.acc, i);
@@ -327,7 +336,18 @@ __global__ void __launch_bounds__(kConsThreads) conservation_kernel(const double
 
 // Threads per block of the per-body kernels: 256, or 64 where that leaves SMs
 // without a block.
-int step_block(int64_t n) { return n < 148 * 256 ? 64 : 256; }
+constexpr int64_t kFewBodies = 148 * 256;
+int step_block(int64_t n) { return n < kFewBodies ? 64 : 256; }
+
+// Calls f with the place of a's sums as a template argument.
+template <class F>
+void with_source(const StepArgs& a, F f) {
+    if (a.fx) f(std::integral_constant<Src, Src::kFx>{});
+    else if (a.f64) f(std::integral_constant<Src, Src::kF64>{});
+    else if (a.tiles) f(std::integral_constant<Src, Src::kTiles>{});
+    else if (a.n < kFewBodies) f(std::integral_constant<Src, Src::kFewSlots>{});
+    else f(std::integral_constant<Src, Src::kSlots>{});
+}
 
 int grid_for(int64_t n, int block) {
     int64_t g = (n + block - 1) / block;
@@ -346,13 +366,15 @@ cudaError_t launch_predictor(const StepArgs& a, cudaStream_t s) {
 
 cudaError_t launch_corrector(const StepArgs& a, cudaStream_t s) {
     const int b = step_block(a.n);
-    corrector_kernel<<<grid_for(a.n, b), b, 0, s>>>(a);
+    with_source(a, [&](auto src) { corrector_kernel<decltype(src)::value><<<grid_for(a.n, b), b, 0, s>>>(a); });
     return cudaGetLastError();
 }
 
 cudaError_t launch_collect(const StepArgs& a, bool want_acc, bool accumulate, cudaStream_t s) {
     const int b = step_block(a.n);
-    collect_kernel<<<grid_for(a.n, b), b, 0, s>>>(a, want_acc ? 1 : 0, accumulate ? 1 : 0);
+    with_source(a, [&](auto src) {
+        collect_kernel<decltype(src)::value><<<grid_for(a.n, b), b, 0, s>>>(a, want_acc ? 1 : 0, accumulate ? 1 : 0);
+    });
     return cudaGetLastError();
 }
 
