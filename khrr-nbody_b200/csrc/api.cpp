@@ -958,6 +958,7 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
         cudaEventCreate(&c->ph0) != cudaSuccess || cudaEventCreate(&c->ph1) != cudaSuccess ||
         c->queue.ensure(kQueueWords) != cudaSuccess || c->kqueue.ensure(kQueueWords) != cudaSuccess ||
         c->errflag.ensure(1) != cudaSuccess || c->cons_done.ensure(1) != cudaSuccess ||
+        c->cic_crowd.ensure(2) != cudaSuccess ||
         c->scratch.ensure(64) != cudaSuccess ||
         take_host_words(&c->host_words) != cudaSuccess) {
         khrr_destroy(c);
@@ -967,6 +968,7 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
     cudaMemset(c->queue.p, 0, kQueueWords * sizeof(unsigned));
     cudaMemset(c->errflag.p, 0, sizeof(unsigned));
     cudaMemset(c->cons_done.p, 0, sizeof(unsigned));
+    cudaMemset(c->cic_crowd.p, 0, 2 * sizeof(unsigned));
     for (int i = 0; i < force_variant_count() + pair_variant_count(); ++i) {
         const ForceVariant* v = i < force_variant_count() ? force_variant(i) : pair_variant(i - force_variant_count());
         if (cudaFuncSetAttribute(v->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -401,10 +401,11 @@ cudaError_t launch_to_float(const double* src, float* dst, int64_t n, cudaStream
 // cell ids as the binning's.  The deposit adds m w into cell_mass (FP64
 // atomics); the gather writes acc = sum w cell_acc and value = sum w
 // cell_value (either output may be NULL), corners in z, y, x order.
-// With copies (ncopies extra meshes, all zero before and after), the blocks
-// take turns at the mesh and its copies, which are then added up.
+// With copies (ncopies extra meshes, all zero before and after, as the two words
+// of crowd are), blocks whose bodies crowd take turns at the mesh and its copies,
+// which are then added up.
 cudaError_t launch_cic_deposit(const double* pos, const double* mass, int64_t n, const MeshGeom& m, double* cell_mass,
-                               double* copies, int ncopies, cudaStream_t s);
+                               double* copies, int ncopies, unsigned* crowd, cudaStream_t s);
 // How many copies pay for n bodies on a mesh.
 int cic_copy_count(int64_t n, int64_t cells);
 cudaError_t launch_cic_gather(const double* pos, int64_t n, const MeshGeom& m, const double* cell_acc,

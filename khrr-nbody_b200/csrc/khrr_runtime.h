@@ -221,6 +221,7 @@ struct khrr_ctx {
     khrr::DevBuf<int> morder;                            // khrr_sort_by_cell: n body indices
     khrr::DevBuf<double> cell_mass, cell_phi, wave_resid;
     khrr::DevBuf<double> cic_copies;                     // khrr_cic_deposit's extra meshes, zero between calls
+    khrr::DevBuf<unsigned> cic_crowd;                    // launch_cic_deposit's two words (the mesh solver's too)
     bool cic_deposited = false;                          // a deposit was made without them
     size_t cic_refused = ~size_t(0);                     // words that the device had no room for (asked once)
     int64_t cell_phi_cells = 0;                          // mesh size the cell_phi sums belong to

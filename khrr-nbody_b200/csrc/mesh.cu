@@ -1107,47 +1107,122 @@ __device__ __forceinline__ CicAxis cic_axis(double p, double lo, double cs, doub
 // at 32^3; 168 -> 111 for 2.1 M bodies at 256^3.  Eight lanes per body, a
 // corner each and the axes shared by shuffles, execute more instructions than
 // that saves (147, and 138 for the gather).
+//
+// With extra meshes (ncopies > 0) the chunks of 128 bodies take turns at them and
+// the mesh.  JUDGE: only if the bodies crowd: of 256 taken evenly from the array,
+// kCrowded or more lie in the cell of an earlier one (32,640 / cells expected of
+// evenly spread bodies, 1.0 at 32^3 and 0.1 at 64^3; a galaxy has 150 there and 24
+// at 128^3).  Every block judges for itself, once for all its chunks, and one that
+// spreads says so to the combining kernel in crowd[0].  (One wave of blocks
+// that judge and later ones that read the word: the reads wait behind the crowded
+// cells' reductions at L2, 51 us for the encounter of 400,000 on 80^3 instead of 33;
+// a block for every chunk: 43 us for 786,432 evenly spread on 128^3 instead of 32.)
+constexpr int kCrowded = 4, kCrowdSlots = 1024;
+constexpr unsigned kJudgeBlocks = 148 * 16;  // two waves: 53.4 us for a galaxy of 786,432 on 128^3, one wave 55.7
+
+template <bool JUDGE>
 __global__ void __launch_bounds__(256) cic_deposit_kernel(const double* __restrict__ pos,
                                                           const double* __restrict__ mass, int64_t n, const MeshGeom m,
                                                           double* __restrict__ cell_mass, double* __restrict__ copies,
-                                                          int ncopies, int64_t cells) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, i = t >> 1;
-    if (i >= n) return;
-    const int a = static_cast<int>(t & 1);
-    const int own = static_cast<int>(blockIdx.x % static_cast<unsigned>(ncopies + 1));
-    double* const out = own == 0 ? cell_mass : copies + (own - 1) * cells;
-    const CicAxis ax = cic_axis(pos[3 * i], m.lo[0], m.cs[0], m.rcs[0], m.g[0]);
-    const CicAxis ay = cic_axis(pos[3 * i + 1], m.lo[1], m.cs[1], m.rcs[1], m.g[1]);
-    const CicAxis az = cic_axis(pos[3 * i + 2], m.lo[2], m.cs[2], m.rcs[2], m.g[2]);
-    const double mi = mass[i];
-    const int x = ax.i0 + a;
-    if (x < 0 || x >= m.g[0]) return;
-    const double wx = a ? ax.w[1] : ax.w[0];
+                                                          int ncopies, int64_t cells, unsigned* __restrict__ crowd) {
+    // The combining kernel is launched behind this one at once, and waits.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    int meshes = ncopies + 1;
+    if constexpr (JUDGE) {
+        __shared__ unsigned seen[kCrowdSlots];
+        const int64_t q = n >= 256 ? threadIdx.x * (n / 256) : threadIdx.x < n ? threadIdx.x : 0;
+        const int x = cic_axis(pos[3 * q], m.lo[0], m.cs[0], m.rcs[0], m.g[0]).i0;
+        const int y = cic_axis(pos[3 * q + 1], m.lo[1], m.cs[1], m.rcs[1], m.g[1]).i0;
+        const int z = cic_axis(pos[3 * q + 2], m.lo[2], m.cs[2], m.rcs[2], m.g[2]).i0;
+        for (int k = threadIdx.x; k < kCrowdSlots; k += 256) seen[k] = ~0u;
+        __syncthreads();
+        bool again = false;
+        if (threadIdx.x < n && x >= -1 && x < m.g[0] && y >= -1 && y < m.g[1] && z >= -1 && z < m.g[2]) {
+            const unsigned cell = ((static_cast<unsigned>(z + 1) * static_cast<unsigned>(m.g[1] + 1) +
+                                    static_cast<unsigned>(y + 1)) * static_cast<unsigned>(m.g[0] + 1) +
+                                   static_cast<unsigned>(x + 1)) & 0x7fffffffu;
+            again = atomicCAS(&seen[(cell * 2654435761u) >> 22], ~0u, cell) == cell;
+        }
+        // Where two of the sample's cells share a slot, the count depends on which
+        // came first: the blocks may differ at the line, so each speaks for itself.
+        if (__syncthreads_count(again) < kCrowded) meshes = 1;
+        else if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned*>(crowd) = 1u;
+    }
+    const int a = threadIdx.x & 1;
+    for (int64_t chunk = blockIdx.x; chunk * 128 < n; chunk += gridDim.x) {
+        const int64_t i = chunk * 128 + (threadIdx.x >> 1);
+        if (i >= n) break;
+        const CicAxis ax = cic_axis(pos[3 * i], m.lo[0], m.cs[0], m.rcs[0], m.g[0]);
+        const CicAxis ay = cic_axis(pos[3 * i + 1], m.lo[1], m.cs[1], m.rcs[1], m.g[1]);
+        const CicAxis az = cic_axis(pos[3 * i + 2], m.lo[2], m.cs[2], m.rcs[2], m.g[2]);
+        const double mi = mass[i];
+        const int own = static_cast<int>(static_cast<unsigned>(chunk) % static_cast<unsigned>(meshes));
+        double* const out = own == 0 ? cell_mass : copies + (own - 1) * cells;
+        const int x = ax.i0 + a;
+        if (x < 0 || x >= m.g[0]) continue;
+        const double wx = a ? ax.w[1] : ax.w[0];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const int z = az.i0 + c;
-        if (z < 0 || z >= m.g[2]) continue;
+        for (int c = 0; c < 2; ++c) {
+            const int z = az.i0 + c;
+            if (z < 0 || z >= m.g[2]) continue;
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const int y = ay.i0 + b;
-            if (y < 0 || y >= m.g[1]) continue;
-            const double w = (wx * ay.w[b]) * az.w[c];
-            atomicAdd(&out[static_cast<int64_t>(z) * m.g[0] * m.g[1] + static_cast<int64_t>(y) * m.g[2] + x], mi * w);
+            for (int b = 0; b < 2; ++b) {
+                const int y = ay.i0 + b;
+                if (y < 0 || y >= m.g[1]) continue;
+                const double w = (wx * ay.w[b]) * az.w[c];
+                atomicAdd(&out[static_cast<int64_t>(z) * m.g[0] * m.g[1] + static_cast<int64_t>(y) * m.g[2] + x], mi * w);
+            }
         }
     }
 }
 
-// The copies' sums into the cells, the copies zero again.
+// The copies' sums into the cells, the copies zero again: U cells of a thread at
+// a time, K copies ahead.  Cells without a sum are only read (a galaxy leaves
+// most of them empty), and the others added to atomically: another deposit of
+// the caller's into the same mesh may be under way.
+template <int U, int K>
+__device__ __forceinline__ void cic_add_copies(double* __restrict__ cell_mass, double* __restrict__ copies, int ncopies,
+                                               int64_t cells) {
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t c0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c0 < cells; c0 += U * stride) {
+        double s[U] = {};
+        for (int k0 = 0; k0 < ncopies; k0 += K) {
+            double v[U][K];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const int64_t c = c0 + u * stride;
+                    v[u][k] = c < cells && k0 + k < ncopies ? copies[(k0 + k) * cells + c] : 0.0;
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    if (v[u][k] != 0.0) {  // true for a NaN as well
+                        s[u] += v[u][k];
+                        copies[(k0 + k) * cells + c0 + u * stride] = 0.0;
+                    }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (s[u] != 0.0) atomicAdd(cell_mass + c0 + u * stride, s[u]);
+    }
+}
+
+// The above if any block spread.  crowd[1] counts the blocks that are done; the
+// last one clears crowd[0].
 __global__ void __launch_bounds__(256) cic_combine_kernel(double* __restrict__ cell_mass, double* __restrict__ copies,
-                                                          int ncopies, int64_t cells) {
-    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (c >= cells) return;
-    double s = 0.0;
-#pragma unroll 4
-    for (int k = 0; k < ncopies; ++k) s += copies[k * cells + c];
-    cell_mass[c] += s;
-#pragma unroll 4
-    for (int k = 0; k < ncopies; ++k) copies[k * cells + c] = 0.0;
+                                                          int ncopies, bool always, int64_t cells,
+                                                          unsigned* __restrict__ crowd) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!always && *reinterpret_cast<volatile unsigned*>(crowd) == 0u) return;
+    if (ncopies <= 2) cic_add_copies<4, 2>(cell_mass, copies, ncopies, cells);
+    else cic_add_copies<1, 8>(cell_mass, copies, ncopies, cells);
+    if (always) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicInc(crowd + 1, gridDim.x - 1) == gridDim.x - 1)
+        *reinterpret_cast<volatile unsigned*>(crowd) = 0u;
 }
 
 // Interpolation back to a body by its two lanes (a: the lane's x corner): acc
@@ -1528,26 +1603,44 @@ cudaError_t launch_deinterleave(const int2* pci, int64_t n, int* a, int* b, cuda
 // sectors one after another, 15 ns each (564 us for a 786,432-body galaxy on
 // 32^3 cells over [-4, 4]^3, where its uniform share would take 20), and with
 // R meshes R of them proceed at once.  Adding the copies up costs R cells of
-// reads and writes, so R goes with the bodies per cell and the meshes stay
-// within 69 MB.  Measured (us, one mesh -> with copies): 786,432 bodies 32^3
-// 564 -> 77, 64^3 209 -> 56, 96^3 146 -> 56, 128^3 68 -> 53; 2 M on 32^3 1428 ->
-// 180, on 160^3 211 -> 164; 20,000 on 32^3 23 -> 13, on 48^3 10 -> 15 (one mesh
-// kept).  Uniformly spread bodies pay for it: 23 -> 31 at 64^3, 21 -> 37 at
-// 128^3.
+// reads, so R goes with the bodies per cell and the meshes stay within 69 MB.
+// Measured (us, one lane per body and one mesh / as it is): a galaxy of 786,432
+// on 32^3 736 / 80, 64^3 302 / 41, 96^3 204 / 62, 128^3 103 / 53; 20,000 on 32^3
+// 23 / 10.  The same evenly spread: 43 / 25, 33 / 29, 33 / 32, 33 / 32; 6.5 / 9.6.
 int cic_copy_count(int64_t n, int64_t cells) {
     const int64_t meshes = std::min<int64_t>({16, 8 * n / cells, int64_t(8600000) / cells});
     return meshes < 2 ? 0 : static_cast<int>(meshes) - 1;
 }
 
 cudaError_t launch_cic_deposit(const double* pos, const double* mass, int64_t n, const MeshGeom& m, double* cell_mass,
-                               double* copies, int ncopies, cudaStream_t s) {
+                               double* copies, int ncopies, unsigned* crowd, cudaStream_t s) {
     if (n < 1) return cudaSuccess;
     const int64_t cells = static_cast<int64_t>(m.g[0]) * m.g[1] * m.g[2];
-    cic_deposit_kernel<<<static_cast<unsigned>((2 * n + 255) / 256), 256, 0, s>>>(pos, mass, n, m, cell_mass, copies,
-                                                                                  ncopies, cells);
-    if (ncopies > 0)
-        cic_combine_kernel<<<static_cast<unsigned>((cells + 255) / 256), 256, 0, s>>>(cell_mass, copies, ncopies, cells);
-    return cudaGetLastError();
+    // Where there are many bodies to a cell, or the meshes are small, judging costs
+    // a galaxy more than it saves evenly spread bodies (us, judged / always: 786,432
+    // on 64^3 47.5 / 41.2 and 28.0 / 28.9, on 32^3 evenly spread 35.0 / 24.8; 100,000
+    // on 64^3 22.7 / 16.6 and 10.4 / 9.4).
+    const bool always = n >= 3 * cells || ncopies * cells <= int64_t(1) << 21;
+    const unsigned chunks = static_cast<unsigned>((n + 127) / 128);
+    if (ncopies > 0 && !always)
+        cic_deposit_kernel<true><<<std::min(chunks, kJudgeBlocks), 256, 0, s>>>(pos, mass, n, m, cell_mass, copies, ncopies,
+                                                                                cells, crowd);
+    else
+        cic_deposit_kernel<false><<<chunks, 256, 0, s>>>(pos, mass, n, m, cell_mass, copies, ncopies, cells, crowd);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || ncopies < 1) return e;
+    // Launched with programmatic stream serialization: where no block spread,
+    // the deposit's end is all that it adds to.
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(std::min<int64_t>((cells + 255) / 256, 148 * 8)));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, cic_combine_kernel, cell_mass, copies, ncopies, always, cells, crowd);
 }
 
 cudaError_t launch_cic_gather(const double* pos, int64_t n, const MeshGeom& m, const double* cell_acc,

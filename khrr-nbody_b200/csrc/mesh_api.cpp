@@ -515,7 +515,8 @@ khrr_status khrr_cic_deposit(khrr_ctx* c, const double* pos, const double* mass,
             }
         }
     }
-    return c->cuda(launch_cic_deposit(pos, mass, n, g, cell_mass, c->cic_copies.p, copies, c->stream), "cic deposit");
+    return c->cuda(launch_cic_deposit(pos, mass, n, g, cell_mass, c->cic_copies.p, copies, c->cic_crowd.p, c->stream),
+                   "cic deposit");
 }
 
 khrr_status khrr_cic_gather(khrr_ctx* c, const double* pos, int64_t n, const khrr_mesh* mesh, const double* cell_acc,
@@ -679,7 +680,8 @@ khrr_status khrr_ctx::mesh_enqueue_force(const double* x, int iters, int rot0) {
     if ((st = cuda(cudaMemsetAsync(M.cell_mass.p, 0, cz * sizeof(double), s), "memset")) != KHRR_OK) return st;
     for (size_t k = 0; k < cnt.size(); ++k) {
         const int64_t o = poff[k];
-        cudaError_t e = cic ? launch_cic_deposit(x + 3 * o, mass.p + o, cnt[k], M.geom, M.cell_mass.p, M.copies.p, M.ncopies, s)
+        cudaError_t e = cic ? launch_cic_deposit(x + 3 * o, mass.p + o, cnt[k], M.geom, M.cell_mass.p, M.copies.p, M.ncopies,
+                                                 cic_crowd.p, s)
                             : launch_assign_cells(x + 3 * o, cnt[k], M.geom, M.pci.p + o, mass.p + o, M.cell_mass.p, s);
         if ((st = cuda(e, "deposit")) != KHRR_OK) return st;
     }
