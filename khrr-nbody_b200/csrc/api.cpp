@@ -836,10 +836,20 @@ khrr_status khrr_ctx::get_step_graph(double dt, int nsteps, int mode, bool phi_l
     const auto key = std::make_tuple(dt_bits, nsteps, mode, phi_last, compat, timing);
     auto it = graphs.find(key);
     if (it != graphs.end()) {
+        it->second.used = ++graph_clock;
         *out = &it->second;
         return KHRR_OK;
     }
+    if (graphs.size() >= kMaxGraphs) {
+        auto old = std::min_element(graphs.begin(), graphs.end(),
+                                    [](const auto& x, const auto& y) { return x.second.used < y.second.used; });
+        // One still running is freed when it has ended.
+        cudaGraphExecDestroy(old->second.exec);
+        cudaGraphDestroy(old->second.graph);
+        graphs.erase(old);
+    }
     StepGraph g{};
+    g.used = ++graph_clock;
     if ((st = cuda(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture")) != KHRR_OK)
         return st;
     khrr_status est = KHRR_OK;

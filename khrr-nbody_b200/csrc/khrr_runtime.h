@@ -119,6 +119,7 @@ struct StepGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaGraphNode_t ev0 = nullptr, ev1 = nullptr;  // event-record nodes around the force pass
+    uint64_t used = 0;  // when it was last asked for (step graphs)
 };
 
 // The mesh-force solver (khrr_set_mesh_solver): its mesh, field ring and
@@ -189,7 +190,12 @@ struct khrr_ctx {
     khrr::ForcePlan plan_batched, plan_plain, plan_fp64;
     bool predicted = false;
     double pred_dt = 0.0;
-    std::map<std::tuple<uint64_t, int, int, bool, bool, bool>, khrr::StepGraph> graphs;  // (dt, steps, mode, phi, compat, timed)
+    // (dt, steps, mode, phi, compat, timed) -> graph: the kMaxGraphs asked for last.  A
+    // program that changes dt with every call would keep 0.16 MB of device and of
+    // host memory for each of them; one of a constant dt has two to four.
+    static constexpr size_t kMaxGraphs = 32;
+    std::map<std::tuple<uint64_t, int, int, bool, bool, bool>, khrr::StepGraph> graphs;
+    uint64_t graph_clock = 0;
     // Every force pass starts from a zero queue counter and, where its kernel
     // accumulates, zero sums; the kernel that reads the sums zeroes both again.
     // clean: the kind of pass they are zero for (0: unknown).
