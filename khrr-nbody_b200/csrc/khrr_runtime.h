@@ -167,8 +167,13 @@ struct khrr_ctx {
     khrr::DevBuf<float> shadow_buf;  // SoA FP32 shadow, 5 x npad
     khrr::DevBuf<double4> part;
     khrr::DevBuf<unsigned long long> fx;  // the pair kernel's fixed-point sums, kFxComps x npad
-    khrr::DevBuf<khrr::FxScale> fx_scale; // their scale per 128-body tile
-    std::vector<khrr::FxScale> fx_scales; // host copy (kept alive until the upload's copies complete)
+    // What an upload finds out per 128-body tile, in one buffer and one copy (3 us
+    // each): the scales of the fixed-point sums, {mass, eps2 / 2} of a tile of 128 real
+    // bodies that share both (else {0, -1}), and the first mass in FP32.
+    khrr::DevBuf<double> tile_info;
+    khrr::FxScale* fx_scale = nullptr;
+    double2* tile_class64 = nullptr;
+    float* tile_mass = nullptr;
     khrr::DevBuf<double> f64_sums;  // the symmetric FP64 pass's sums, 2 x 4 x npad
     khrr::DevBuf<unsigned> queue, errflag;
     // Page-locked words that small results come back through: 16 doubles of
@@ -181,8 +186,6 @@ struct khrr_ctx {
     bool uniform = false;
     float h_uniform = 0.0f;
     bool tile_uniform_mass = false;     // every 128-body tile of the layout has one mass
-    khrr::DevBuf<float> tile_mass;      // that mass per tile (FP32)
-    khrr::DevBuf<double2> tile_class64; // per tile {mass, eps2 / 2} of a tile of 128 real bodies that share both, else {0, -1}
     bool block_uniform_mass = false;    // every pair block has one mass (the pair kernel's block-mass form)
     khrr::PairBlocks pair_blocks;       // the pair kernel's blocks of the layout
     khrr::FieldConsts field{};
