@@ -10,6 +10,7 @@
 // kernels read the FP32 structure-of-arrays shadow (x, y, z, m, eps2 / 2); the
 // one-sided kernel writes FP64 partials part[slot][body], the symmetric pair
 // kernel adds into 64-bit fixed-point sums fx[component][body].
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -19,7 +20,6 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
-#include <mutex>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -36,46 +36,49 @@ using namespace khrr;
 // ---------------------------------------------------------------------------
 namespace {
 
-// Page-locked words for contexts, kHostWords doubles each.  Allocating and
-// freeing page-locked memory takes 2 ms or more, a context's creation without
-// it 3 ms: the slots of one page, kept for the process, serve up to 16 contexts
-// at a time, and any more allocate their own.
-constexpr size_t kHostWords = 32, kHostSlots = 16;
-std::mutex host_page_mutex;
-double* host_page = nullptr;
-unsigned host_page_used = 0;  // one bit per slot
+// The pool's allocator: the runtime's, and the identity of the device's primary
+// context from the driver (the library does not link libcuda directly), which a
+// reset of the device changes.
+struct HostWordApi {
+    cudaError_t last = cudaSuccess;
+    int epoch(int device, uint64_t* id) {
+        static const PFN_cuCtxGetId_v12000 get = [] {
+            void* p = nullptr;
+            cudaDriverEntryPointQueryResult q{};
+            if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
+                q != cudaDriverEntryPointSuccess)
+                p = nullptr;
+            return reinterpret_cast<PFN_cuCtxGetId_v12000>(p);
+        }();
+        unsigned long long v = 0;
+        if ((last = cudaSetDevice(device)) != cudaSuccess) return 1;
+        if (!get || get(nullptr, &v) != CUDA_SUCCESS) return 1;
+        *id = v;
+        return 0;
+    }
+    int alloc(double** p, size_t n) {
+        last = cudaHostAlloc(reinterpret_cast<void**>(p), n * sizeof(double), cudaHostAllocPortable);
+        return last != cudaSuccess;
+    }
+    int free(double* p) {
+        last = cudaFreeHost(p);
+        return last != cudaSuccess;
+    }
+};
 
-cudaError_t take_host_words(double** out) {
-    std::lock_guard<std::mutex> lock(host_page_mutex);
-    cudaPointerAttributes at{};
-    if (host_page && (cudaPointerGetAttributes(&at, host_page) != cudaSuccess || at.type != cudaMemoryTypeHost)) {
-        (void)cudaGetLastError();  // the program reset its device: the page is gone
-        host_page = nullptr;
-        host_page_used = 0;
-    }
-    if (!host_page) {
-        const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&host_page),
-                                            kHostSlots * kHostWords * sizeof(double), cudaHostAllocPortable);
-        if (e != cudaSuccess) {
-            host_page = nullptr;
-            return e;
-        }
-    }
-    for (size_t k = 0; k < kHostSlots; ++k)
-        if (!(host_page_used >> k & 1u)) {
-            host_page_used |= 1u << k;
-            *out = host_page + k * kHostWords;
-            return cudaSuccess;
-        }
-    return cudaHostAlloc(reinterpret_cast<void**>(out), kHostWords * sizeof(double), cudaHostAllocPortable);
+HostWordPool<HostWordApi>& host_word_pool() {
+    static HostWordPool<HostWordApi>* const pool = new HostWordPool<HostWordApi>();  // outlives static contexts
+    return *pool;
 }
 
-// After the context's last work on its stream has ended.
-void give_host_words(double* p) {
-    std::lock_guard<std::mutex> lock(host_page_mutex);
-    if (host_page && p >= host_page && p < host_page + kHostSlots * kHostWords)
-        host_page_used &= ~(1u << ((p - host_page) / kHostWords));
-    else cudaFreeHost(p);
+bool take_host_words(int device, HostWords* out) {
+    HostWordApi api;
+    return host_word_pool().take(api, device, out) == 0;
+}
+
+void give_host_words(const HostWords& w) {
+    HostWordApi api;
+    host_word_pool().give(api, w);
 }
 
 int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
@@ -973,10 +976,11 @@ khrr_status khrr_create(int device, khrr_ctx** out) {
         c->errflag.ensure(1) != cudaSuccess || c->cons_done.ensure(1) != cudaSuccess ||
         c->cic_crowd.ensure(2) != cudaSuccess ||
         c->scratch.ensure(64) != cudaSuccess ||
-        take_host_words(&c->host_words) != cudaSuccess) {
+        !take_host_words(device, &c->words)) {
         khrr_destroy(c);
         return KHRR_ERR_CUDA;
     }
+    c->host_words = c->words.p;
     c->stream = c->own;
     cudaMemset(c->queue.p, 0, kQueueWords * sizeof(unsigned));
     cudaMemset(c->errflag.p, 0, sizeof(unsigned));
@@ -1013,9 +1017,9 @@ void khrr_destroy(khrr_ctx* c) {
     if (c->ph0) cudaEventDestroy(c->ph0);
     if (c->ph1) cudaEventDestroy(c->ph1);
     if (c->own) cudaStreamDestroy(c->own);
-    double* words = c->host_words;
+    const HostWords words = c->words;
     delete c;  // device buffers free themselves, after the device's work
-    if (words) give_host_words(words);
+    give_host_words(words);
 }
 
 const char* khrr_last_error(const khrr_ctx* c) { return c ? c->err.c_str() : "null context"; }

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "khrr.h"
+#include "host_words.h"
 #include "khrr_internal.h"
 
 namespace khrr {
@@ -179,7 +180,8 @@ struct khrr_ctx {
     // Page-locked words that small results come back through: 16 doubles of
     // khrr_conservation (the last one the error flag's value), then the error
     // flag of khrr_synchronize.  Read by the host after a synchronisation.
-    double* host_words = nullptr;
+    khrr::HostWords words;
+    double* host_words = nullptr;  // words.p
     khrr_status report_flag(unsigned flag);
     khrr::DevBuf<double> cons_blocks, scratch;
     khrr::DevBuf<unsigned> cons_done;  // khrr_conservation's count of finished blocks (zero between calls)
