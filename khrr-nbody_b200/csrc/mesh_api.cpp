@@ -504,7 +504,13 @@ khrr_status khrr_cic_deposit(khrr_ctx* c, const double* pos, const double* mass,
             c->cic_deposited = true;
             copies = 0;
         } else if (c->cic_copies.n < need) {
-            if (c->cic_copies.ensure(need) != cudaSuccess) {
+            // A deposit needs no allocation otherwise, and may be made while the
+            // thread captures another stream: it must not end that capture.
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            if ((st = c->cuda(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode")) != KHRR_OK) return st;
+            const cudaError_t e = c->cic_copies.ensure(need);
+            if ((st = c->cuda(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode")) != KHRR_OK) return st;
+            if (e != cudaSuccess) {
                 (void)cudaGetLastError();  // no room: deposit directly
                 c->cic_refused = need;
                 copies = 0;
