@@ -16,7 +16,8 @@ for both bodies, so it executes fewer than 20 per interaction).
 N > 1 (under torchrun) runs N independent replicas (the path is pinned to one
 GPU per galaxy; there is no data-path collective), timed as the max over ranks.
 --impl reference times the reference's own ACCEL_kernel compiled for the host
-(oracle/_ref, OpenMP over all host threads) on a bounded target sample.
+(oracle/_ref, OpenMP over all host threads) on a bounded target sample; without
+that build it says that it is unavailable.
 """
 from __future__ import annotations
 
@@ -223,6 +224,15 @@ def cpu_reference_sample(pos, vel, mass, eps2, seconds, rng):
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return 0
+    sys.path.insert(0, str(ROOT / "oracle"))
+    import pyoracle
+    try:
+        pyoracle.Reference()
+    except FileNotFoundError:
+        # The oracle's restatement is not the reference: no number of its.
+        print(json.dumps({"impl": "reference", "unavailable": "its host build (oracle/_ref) is absent: the reference's "
+                                                              "sources are not on this machine"}), flush=True)
         return 0
     pos, vel, mass, eps2 = workload(args.n_stars, args.n_dm)
     rng = np.random.default_rng(7)
