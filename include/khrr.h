@@ -233,7 +233,10 @@ enum {
  * spreads its mass over the 8 cells around u = (x - lo)/cell - 1/2 with
  * weights (1 - f, f) per axis (f = u - floor(u)); corners outside the mesh
  * are dropped.  Device pointers: pos n double3, mass n, cell_mass C
- * (accumulated into, FP64 atomics).  Cubic meshes only. */
+ * (accumulated into, FP64 atomics).  Cubic meshes only.  From its second deposit
+ * on a context spreads crowded bodies over up to 15 extra meshes, at most 69 MB,
+ * which it keeps (none where the device has no room, and none in a capture of the
+ * caller's); the mesh solver has its own. */
 khrr_status khrr_cic_deposit(khrr_ctx* ctx, const double* pos, const double* mass, int64_t n,
                              const khrr_mesh* mesh, double* cell_mass);
 /* Cloud-in-cell interpolation, the gather matching khrr_cic_deposit (the
@@ -388,7 +391,8 @@ khrr_status khrr_accel_fp64_sample(khrr_ctx* ctx, const int64_t* targets, int64_
  * KHRR_FP64; KHRR_MESH). */
 khrr_status khrr_forces(khrr_ctx* ctx, int flags);
 /* nsteps predictor -> force -> corrector steps of size dt (nbody.cu:1525-1582),
- * replayed from a CUDA graph.  flags: KHRR_PHI evaluates the potential at the
+ * replayed from CUDA graphs of up to eight steps, of which a context keeps the 32
+ * used last (one per dt, step count and flags).  flags: KHRR_PHI evaluates the potential at the
  * new positions in the last step's force pass; KHRR_COMPAT_ACCUMULATE;
  * KHRR_PLAIN (per-system launches) or KHRR_FP64 (the FP64 direct sum);
  * KHRR_MESH. */

@@ -4,7 +4,7 @@
 // its energy drift against this path.
 //
 // Two forms.  fp64_pair_kernel (the default; below) evaluates each unordered
-// pair once for both bodies on the FP32 pair kernel's plan.  fp64_force_kernel
+// pair once for both bodies on the tapered plan of single tiles.  fp64_force_kernel
 // (KHRR_FP64_ONESIDED=1) evaluates every ordered pair: the one-sided
 // kernel's queue of WorkItems (system, i tile of 512 bodies, j chunk),
 // pulled by a persistent grid with one atomic per item; each item writes its
@@ -128,12 +128,12 @@ __global__ void __launch_bounds__(NT, kMinCtas) fp64_force_kernel(const F64Args 
 }
 
 // The symmetric form of the same sums (the default FP64 pass): every
-// unordered pair of a system evaluated once for both bodies, on the FP32
-// pair kernel's work plan (1024-body blocks, a block row cut into chunks of
-// 128-body tiles, the block's own tiles one-sided).  A CTA holds its i block
-// in registers (128 threads x 8 bodies) and streams the chunk's j tiles of
-// 128 bodies through a double-buffered shared-memory tile; the reaction on a
-// j body is summed across a warp by handing it from lane to lane (lane l
+// unordered pair of a system evaluated once for both bodies, on a plan of its
+// own (plan_pair_tiles: 1024-body blocks, a block row cut into chunks of
+// 128-body tiles that taper to single ones, the block's own tiles one-sided).
+// A CTA holds its i block in registers (128 threads x 8 bodies) and streams the
+// chunk's j tiles of 128 bodies through a double-buffered shared-memory tile; the
+// reaction on a j body is summed across a warp by handing it from lane to lane (lane l
 // evaluates body (l + s) mod 32 of a 32-body sub-chunk at step s and passes
 // its running reaction to lane l - 1), then across the 4 warps in shared
 // memory, and added with FP64 atomics into the body's sums, as are the i
@@ -141,9 +141,9 @@ __global__ void __launch_bounds__(NT, kMinCtas) fp64_force_kernel(const F64Args 
 // throughout; their order differs from the reference's j loop only at the
 // level of FP64 rounding.
 //
-// A body's sum over the partials is kept in two doubles: every partial is cut at a multiple of the body's grid, coarse enough
-// (2^-51 of the bound on its force) that the upper parts add up without
-// rounding, and the lower parts, below 2^-52 of that bound, add up in the
+// A body's sum over the partials is kept in two doubles: every partial is cut
+// at a multiple of the body's grid, coarse enough (2^-51 of the bound on its
+// force) that the upper parts add up without rounding, and the lower parts, below 2^-52 of that bound, add up in the
 // second.  So the number of partials, and the order the atomics land in, do
 // not show in the result: relative RMS error against 80-bit sums 2.4e-16 with
 // one double and chunks of eight tiles, 3.5e-16 with one double and these

@@ -98,14 +98,14 @@ PairBlocks pair_blocks_fixed(const std::vector<int64_t>& poff);
 PairBlocks pair_blocks_by_mass(const std::vector<int64_t>& poff, const std::vector<float>& tile_mass);
 // The pair kernel's items: block rows cut into chunks of `chunk` blocks (0 =
 // chosen from the CTA count), costliest first.
+void plan_pair_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int ctas, int chunk,
+                     ForcePlan& out);
 // The pair plan's work in the small-layout form, or small_ki = 0 (the pair
 // kernel is faster, or its items are not single block pairs).
 void plan_small_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int sms, ForcePlan& out);
 // Time weights of a pair plan's items, heaviest first, and the share of one of
 // `sms` SMs.
 void weigh_pair_items(int sms, ForcePlan& out);
-void plan_pair_items(const PairBlocks& blocks, const std::vector<int64_t>& cnt, int ctas, int chunk,
-                     ForcePlan& out);
 // The same pairs cut at 128-body tiles (1024-body i blocks): chunks taper from
 // a quarter of a CTA's share of the work down to one tile, so layouts of any
 // size fill the persistent grid and its last round.

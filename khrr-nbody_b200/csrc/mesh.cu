@@ -1109,18 +1109,18 @@ __device__ __forceinline__ CicAxis cic_axis(double p, double lo, double cs, doub
 // that saves (147, and 138 for the gather).
 //
 // With extra meshes (ncopies > 0) the chunks of 128 bodies take turns at them and
-// the mesh.  JUDGE: only if the bodies crowd: of 256 taken evenly from the array,
+// the mesh.  SAMPLE: only if the bodies crowd: of 256 taken evenly from the array,
 // kCrowded or more lie in the cell of an earlier one (32,640 / cells expected of
 // evenly spread bodies, 1.0 at 32^3 and 0.1 at 64^3; a galaxy has 150 there and 24
-// at 128^3).  Every block judges for itself, once for all its chunks, and one that
+// at 128^3).  Every block decides for itself, once for all its chunks, and one that
 // spreads says so to the combining kernel in crowd[0].  (One wave of blocks
-// that judge and later ones that read the word: the reads wait behind the crowded
+// that decide and later ones that read the word: the reads wait behind the crowded
 // cells' reductions at L2, 51 us for the encounter of 400,000 on 80^3 instead of 33;
 // a block for every chunk: 43 us for 786,432 evenly spread on 128^3 instead of 32.)
 constexpr int kCrowded = 4, kCrowdSlots = 1024;
-constexpr unsigned kJudgeBlocks = 148 * 16;  // two waves: 53.4 us for a galaxy of 786,432 on 128^3, one wave 55.7
+constexpr unsigned kSampleBlocks = 148 * 16;  // two waves: 53.4 us for a galaxy of 786,432 on 128^3, one wave 55.7
 
-template <bool JUDGE>
+template <bool SAMPLE>
 __global__ void __launch_bounds__(256) cic_deposit_kernel(const double* __restrict__ pos,
                                                           const double* __restrict__ mass, int64_t n, const MeshGeom m,
                                                           double* __restrict__ cell_mass, double* __restrict__ copies,
@@ -1128,7 +1128,7 @@ __global__ void __launch_bounds__(256) cic_deposit_kernel(const double* __restri
     // The combining kernel is launched behind this one at once, and waits.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     int meshes = ncopies + 1;
-    if constexpr (JUDGE) {
+    if constexpr (SAMPLE) {
         __shared__ unsigned seen[kCrowdSlots];
         const int64_t q = n >= 256 ? threadIdx.x * (n / 256) : threadIdx.x < n ? threadIdx.x : 0;
         const int x = cic_axis(pos[3 * q], m.lo[0], m.cs[0], m.rcs[0], m.g[0]).i0;
@@ -1431,8 +1431,10 @@ cudaError_t launch_wave_f64(double* phi_new, const double* phi, const double* ph
                           reinterpret_cast<uintptr_t>(phi_old) | reinterpret_cast<uintptr_t>(mass);
     if (w.nx % 2 == 0 && any % 16 == 0 && w.nx >= 178 && w.nx <= 352) {
         // The planes through shared memory where the field does not stay in L2:
-        // us per iteration, march / this, 33.6 / 30.9 at 170^3, 35.1 / 36.8 at
-        // 176^3, 39.4 / 35.1 at 180^3, 51.7 / 45.6 at 200^3, 255.8 / 217.1 at
+        // us per iteration, march / this, 27.3 / 31.5 at 160^3, 30.9 / 33.1 at
+        // 164^3, 31.9 / 33.5 at 168^3, 33.8 / 31.4 at 170^3 (the one size below the
+        // line whose cut fills the chip), 34.7 / 36.1 at 172^3, 35.2 / 37.0 at
+        // 176^3, 39.4 / 35.2 at 180^3, 52.1 / 45.3 at 200^3, 255.8 / 217.1 at
         // 350^3, 275.2 / 279.5 at 360^3, 382.3 / 382.7 at 400^3.
         // Segments of 1,280 cells and three stages, or of 1,024 and four: the one
         // whose blocks fill the chip better (us per iteration, 1,280 / 1,024:
@@ -1616,14 +1618,14 @@ cudaError_t launch_cic_deposit(const double* pos, const double* mass, int64_t n,
                                double* copies, int ncopies, unsigned* crowd, cudaStream_t s) {
     if (n < 1) return cudaSuccess;
     const int64_t cells = static_cast<int64_t>(m.g[0]) * m.g[1] * m.g[2];
-    // Where there are many bodies to a cell, or the meshes are small, judging costs
-    // a galaxy more than it saves evenly spread bodies (us, judged / always: 786,432
+    // Where there are many bodies to a cell, or the meshes are small, the sample costs
+    // a galaxy more than it saves evenly spread bodies (us, sampled / always: 786,432
     // on 64^3 47.5 / 41.2 and 28.0 / 28.9, on 32^3 evenly spread 35.0 / 24.8; 100,000
     // on 64^3 22.7 / 16.6 and 10.4 / 9.4).
     const bool always = n >= 3 * cells || ncopies * cells <= int64_t(1) << 21;
     const unsigned chunks = static_cast<unsigned>((n + 127) / 128);
     if (ncopies > 0 && !always)
-        cic_deposit_kernel<true><<<std::min(chunks, kJudgeBlocks), 256, 0, s>>>(pos, mass, n, m, cell_mass, copies, ncopies,
+        cic_deposit_kernel<true><<<std::min(chunks, kSampleBlocks), 256, 0, s>>>(pos, mass, n, m, cell_mass, copies, ncopies,
                                                                                 cells, crowd);
     else
         cic_deposit_kernel<false><<<chunks, 256, 0, s>>>(pos, mass, n, m, cell_mass, copies, ncopies, cells, crowd);

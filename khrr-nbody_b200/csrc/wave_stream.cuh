@@ -8,11 +8,11 @@
 // ST planes.  The neighbours in y and x come from shared memory, the ones in z
 // from registers and from the next stage.
 //
-// What it is for: above 170^3 the march waits for memory with 30 KB an SM on
+// What it is for: from 178^3 on the march waits for memory with 30 KB an SM on
 // the way (640 threads, 48 bytes each); the ring keeps 50 to 100 KB on the way.
-// us per iteration, march / this: 200^3 51.8 / 45.3 (5.7 TB/s of 32 bytes a
-// cell), 240^3 85.6 / 73.8, 256^3 103.2 / 91.2, 320^3 200 / 180.  Below, where the
-// field stays in L2, the march is faster (160^3 27.1 / 29.4).  FP32 gained
+// us per iteration, march / this: 200^3 52.1 / 45.3 (5.7 TB/s of 32 bytes a
+// cell), 240^3 85.6 / 73.8, 256^3 103.6 / 91.2, 320^3 200 / 180.  Below, where the
+// field stays in L2, the march is faster (160^3 27.3 / 31.5).  FP32 gained
 // nothing (256^3 49.1 / 49.3).  Dealing the planes out as equal runs over the
 // grid, so that blocks of neighbouring cells are at different planes, loses the
 // shared rows in L2: 50.3 at 200^3, 82.8 at 240^3.

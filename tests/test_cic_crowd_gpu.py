@@ -1,5 +1,5 @@
 """The cloud-in-cell deposit's choice, on the device, between the mesh and its
-extra meshes: bodies spread evenly, with a few pairs in the sample that it judges
+extra meshes: bodies spread evenly, with a few pairs in the sample that it goes
 by (on both sides of its line), crowded throughout, crowded only in the last
 or the first blocks, sums that cancel, in turns on one context (the extra meshes
 and the words end as they began); and two contexts that deposit into one mesh at
@@ -30,7 +30,7 @@ def bodies(kind, n=N):
         pos[-n // 4:] = rng.uniform(0.13, 0.24, (n - n * 3 // 4, 3))
     elif kind == "crowded at the start":
         pos[:300] = rng.uniform(0.13, 0.24, (300, 3))
-    elif kind.startswith("pairs"):  # of the judged sample's 256 bodies, so many pairs share a place
+    elif kind.startswith("pairs"):  # of the sample's 256 bodies, so many pairs share a place
         k, at = int(kind[-1]), np.arange(256) * (n // 256)
         pos[at[1:2 * k:2]] = pos[at[0:2 * k:2]]
     elif kind == "cancelling":
@@ -43,7 +43,7 @@ def mesh_of(khrr, nx=NX):
     return khrr.Mesh.make((-L,) * 3, (2 * L / nx,) * 3, (nx,) * 3)
 
 
-# 32^3: spread always; 88^3: judged (four extra meshes).
+# 32^3: spread always; 88^3: by the sample (four extra meshes).
 @pytest.mark.parametrize("nx,n", [(NX, N), (88, 500003)])
 def test_kinds_in_turn(khrr_mod, oracle, nx, n):
     import torch
